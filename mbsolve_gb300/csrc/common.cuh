@@ -42,7 +42,6 @@ struct run_desc {
     uint64_t offset;      // global index of the run's cell 0
     uint32_t n_x;
     uint32_t n_t;
-    double dx_inv;
     uint32_t src_begin, src_end;
     uint32_t rec_begin, rec_end;
     // mirror boundary (MBG_BC_MIRROR): H beyond the left end = k_left E[0],

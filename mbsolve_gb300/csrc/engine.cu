@@ -1085,7 +1085,6 @@ private:
             rd.offset = offsets_[r];
             rd.n_x = rs.n_x;
             rd.n_t = rs.n_t;
-            rd.dx_inv = 1.0 / rs.dx;
             rd.k_left = rs.k_left;
             rd.k_right = rs.k_right;
             rd.src_begin = (uint32_t) srcs.size();

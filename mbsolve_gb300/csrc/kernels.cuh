@@ -117,19 +117,39 @@ __device__ __forceinline__ void rot_coeffs<float>(float x, float& s, float& s2)
     }
 }
 
+// FP64: an instruction holds its scheduler's FP64 unit for 64 cycles (one
+// chain of dependent operations or several, one lane or 32: measured), so
+// the count of FP64 instructions is the time of the FP64 kernels. Series in
+// Horner form by compile-time reciprocals (a division takes ten
+// instructions), as many terms as the range needs: for |x| < 2^-9 (the
+// field rotation of a step in the workloads here) the first omitted terms
+// are below 1e-20 of the result, for |x| < 1/4 below 1e-17; 8 and 18
+// instructions. With the 20 divisions of a recurrence before, a 2-level
+// point and step took 193 FP64 instructions; now about 30 (2-level preset,
+// 32,768 points: 1.98e9 -> 8.1e9 cell-updates/s; 6 levels, 65,536 points:
+// 9.5e7 -> 3.2e8, the unit's rate for the 1,225 products of a step).
 template<>
 __device__ __forceinline__ void rot_coeffs<double>(double x, double& s, double& s2)
 {
-    if (fabs(x) < 0.25) {
-        double x2 = x * x;
-        double t = 1.0, u = 1.0;
-#pragma unroll
-        for (int k = 10; k >= 1; k--) {
-            t = 1.0 - x2 / ((2.0 * k) * (2.0 * k + 1.0)) * t;
-            u = 1.0 - x2 / ((2.0 * k + 1.0) * (2.0 * k + 2.0)) * u;
-        }
-        s = x * t;
-        s2 = 0.5 * x2 * u;
+    const double x2 = x * x;
+    if (fabs(x) < 0.001953125) {
+        s = fma(x * x2, fma(x2, 1.0 / 120.0, -1.0 / 6.0), x);
+        s2 = x2 * fma(x2, fma(x2, 1.0 / 720.0, -1.0 / 24.0), 0.5);
+    } else if (fabs(x) < 0.25) {
+        // sin x = x (1 - x^2/3! + ... + x^12/13!)
+        double t = fma(x2, 1.0 / 6227020800.0, -1.0 / 39916800.0);
+        t = fma(x2, t, 1.0 / 362880.0);
+        t = fma(x2, t, -1.0 / 5040.0);
+        t = fma(x2, t, 1.0 / 120.0);
+        t = fma(x2, t, -1.0 / 6.0);
+        s = fma(x * x2, t, x);
+        // 1 - cos x = x^2 (1/2! - x^2/4! + ... + x^12/14!)
+        double u = fma(x2, 1.0 / 87178291200.0, -1.0 / 479001600.0);
+        u = fma(x2, u, 1.0 / 3628800.0);
+        u = fma(x2, u, -1.0 / 40320.0);
+        u = fma(x2, u, 1.0 / 720.0);
+        u = fma(x2, u, -1.0 / 24.0);
+        s2 = x2 * fma(x2, u, 0.5);
     } else {
         double c;
         sincos(x, &s, &c);
@@ -350,14 +370,26 @@ __device__ __forceinline__ void row_dot(const CF& c, const T (&x)[V], T& s, T& s
     }
 }
 
+// Planes the field can rotate for V = N^2 - 1 entries: one per pair of the
+// dipole operator's eigenvalues, N (N - 1) / 2. The V / 2 angles of the
+// material block beyond them are zero (the null space of U has N - 1
+// dimensions at least), their rotations the identity.
+template<int V>
+constexpr int cvr_planes()
+{
+    return V == 3 ? 1 : V == 8 ? 3 : V == 15 ? 6 : V == 24 ? 10 : V == 35 ? 15 : V / 2;
+}
+
 // Coherence-vector step in the plane basis, on the state v kept one half
 // step ahead (see cvr_layout in precompute.cuh): rotate each plane by
-// theta_k dt e; v = v + (Bd v + k); P = p0 + g . v.
-template<typename T, int V, class CF>
+// theta_k dt e; v = v + (Bd v + k); P = p0 + g . v. SP (2 levels): the
+// products with the zeros of cvr2_sparse are left out, 5 of 12.
+template<bool SP = false, typename T, int V, class CF>
 __device__ __forceinline__ void cvr_update(T (&u)[V], T e, T& pout, const CF& cf)
 {
+    static_assert(!SP || V == 3, "sparse form: 2 levels");
     const auto c = cf.pass();
-    static_for<0, V / 2>([&](auto K) {
+    static_for<0, cvr_planes<V>()>([&](auto K) {
         constexpr int k = decltype(K)::value;
         T sn, s2;
         rot_coeffs<T>(c.th(k) * e, sn, s2);
@@ -370,13 +402,22 @@ __device__ __forceinline__ void cvr_update(T (&u)[V], T e, T& pout, const CF& cf
         constexpr int i = decltype(I)::value;
         T sl = T(0);
         s[i] = c.k(i);
-        row_dot<false, i>(c, u, s[i], sl);
+        if constexpr (SP) {
+            if constexpr (i == 1) {
+                s[i] = fma(c.Bd(1, 1), u[1], s[i]);
+            } else {
+                s[i] = fma(c.Bd(i, 0), u[0], s[i]);
+                s[i] = fma(c.Bd(i, 2), u[2], s[i]);
+            }
+        } else {
+            row_dot<false, i>(c, u, s[i], sl);
+        }
     });
     T pp = c.p0();
     static_for<0, V>([&](auto I) {
         constexpr int i = decltype(I)::value;
         u[i] += s[i];
-        pp = fma(c.g(i), u[i], pp);
+        if constexpr (!SP || i != 1) pp = fma(c.g(i), u[i], pp);
     });
     pout = pp;
 }
@@ -398,6 +439,20 @@ __device__ __forceinline__ void df_renorm(float& h, float& l)
     const float s = h + l;
     l = l - (s - h);
     h = s;
+}
+
+// The couplings that the plane basis of a 2-level medium with a diagonal
+// Hamiltonian and a real dipole leaves exactly zero: the field rotates the
+// (0, 1) plane, the free evolution couples 0 and 2 (precession) and relaxes
+// 1 on its own, and P reads 0 and 2. A uniform tile whose block has them
+// zero skips their products (a product with an exact zero changes no sum).
+template<typename T>
+__device__ __forceinline__ bool cvr2_sparse(const T* cb)
+{
+    const cvr_coef<T, 3> c{ cb };
+    return c.Bd(0, 1) == T(0) && c.Bd(1, 0) == T(0) && c.Bd(1, 2) == T(0) && c.Bd(2, 1) == T(0) &&
+        c.Bdl(0, 1) == T(0) && c.Bdl(1, 0) == T(0) && c.Bdl(1, 2) == T(0) && c.Bdl(2, 1) == T(0) &&
+        c.g(1) == T(0);
 }
 
 // Coefficients of the 2-level update held in registers (uniform tiles).
@@ -447,7 +502,7 @@ __device__ __forceinline__ void cvr_update_df(float (&uh)[V], float (&ul)[V], fl
         d[i] = 0.0f;
         r[i] = uh[i];
     });
-    static_for<0, V / 2>([&](auto K) {
+    static_for<0, cvr_planes<V>()>([&](auto K) {
         constexpr int k = decltype(K)::value;
         float sn, s2;
         rot_coeffs<float>(c.th(k) * e, sn, s2);

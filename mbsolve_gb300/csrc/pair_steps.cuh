@@ -55,19 +55,6 @@ struct cvr2_pair_coef {
     }
 };
 
-// The couplings that the plane basis of a 2-level medium with a diagonal
-// Hamiltonian and a real dipole leaves exactly zero: the field rotates the
-// (0, 1) plane, the free evolution couples 0 and 2 (precession) and relaxes
-// 1 on its own, and P reads 0 and 2. A uniform tile whose block has them
-// zero skips their products (a product with an exact zero changes no sum).
-__device__ __forceinline__ bool cvr2_sparse(const float* cb)
-{
-    const cvr_coef<float, 3> c{ cb };
-    return c.Bd(0, 1) == 0.0f && c.Bd(1, 0) == 0.0f && c.Bd(1, 2) == 0.0f && c.Bd(2, 1) == 0.0f &&
-        c.Bdl(0, 1) == 0.0f && c.Bdl(1, 0) == 0.0f && c.Bdl(1, 2) == 0.0f && c.Bdl(2, 1) == 0.0f &&
-        c.g(1) == 0.0f;
-}
-
 // cvr_update_df<3> on two points: the rotation of the (0, 1) plane by
 // theta dt e (rot_coeffs' series, its negated Horner chain for 1 - cos
 // giving the same roundings), the correction k + Bd r with its low-word

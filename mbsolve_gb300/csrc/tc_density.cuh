@@ -277,7 +277,7 @@ struct coef_small {
 template<int V, class CF>
 __device__ __forceinline__ void rotate_df(float (&uh)[V], float (&ul)[V], float e, const CF& cf)
 {
-    static_for<0, V / 2>([&](auto KI) {
+    static_for<0, cvr_planes<V>()>([&](auto KI) {
         constexpr int k = decltype(KI)::value;
         float sn, s2;
         rot_coeffs<float>(cf.th(k) * e, sn, s2);

@@ -79,7 +79,6 @@ __device__ __forceinline__ bool tile_steps(
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const int64_t nx = rd.n_x;
-    const T dxi = (T) rd.dx_inv;
     auto block = [&](int j) -> const T* {
         return UNIFORM ? sh_coef : p.mc + (uint64_t) (M[j] >= 0 ? M[j] : 0) * p.mstride;
     };
@@ -88,6 +87,8 @@ __device__ __forceinline__ bool tile_steps(
     const bool qm_uniform = UNIFORM && sh_coef[pre::FD_HAS_QM] != T(0);
     using creg_t = typename std::conditional<REGCOEF, cvr_coef_reg<T, 3>, no_coef>::type;
     const creg_t creg(sh_coef);
+    bool sparse = false;
+    if constexpr (REGCOEF && !DFD) sparse = cvr2_sparse(sh_coef);
     const int nsrc = tl.overflow ? (int) (rd.src_end - rd.src_begin) : tl.nsrc;
     const int nrec = tl.overflow ? (int) (rd.rec_end - rd.rec_begin) : tl.nrec;
     // Mirror walls are handled only on tiles of the non-uniform path (the
@@ -144,9 +145,9 @@ __device__ __forceinline__ bool tile_steps(
                 const fcoef f = UNIFORM ? fu : load_fcoef(block(j));
                 E[j] = fmaf(f.a, E[j], fmaf(f.bh, hn - H[j], -f.g * P[j]));
             } else {
+                // four FP64 instructions (rot_coeffs<double>: each counts)
                 const T* cb = block(j);
-                E[j] = cb[pre::FD_A] * E[j] +
-                    cb[pre::FD_B] * (-cb[pre::FD_GAMMA] * P[j] + (hn - H[j]) * dxi);
+                E[j] = fma(cb[pre::FD_A], E[j], fma(cb[pre::FD_BDX], hn - H[j], -cb[pre::FD_G] * P[j]));
             }
         }
         // ---- sources, after E and before H (solver_cpu_fdtd.tpp:245-255)
@@ -253,8 +254,10 @@ __device__ __forceinline__ bool tile_steps(
                     if constexpr (REGCOEF) {
                         if constexpr (DFD)
                             cvr_update_df<D>(R[j], Rl[j], e, P[j], creg);
+                        else if (sparse)
+                            cvr_update<true>(R[j], e, P[j], creg);
                         else
-                            cvr_update<T, D>(R[j], e, P[j], creg);
+                            cvr_update(R[j], e, P[j], creg);
                     } else if constexpr (TC) {
                         // mixed tile of the tensor-core kernel: in place
                         // through this thread's row of the idle A operand
@@ -265,13 +268,13 @@ __device__ __forceinline__ bool tile_steps(
                         if constexpr (DFD)
                             cvr_update_df<D>(R[j], Rl[j], e, P[j], cf);
                         else
-                            cvr_update<T, D>(R[j], e, P[j], cf);
+                            cvr_update(R[j], e, P[j], cf);
                     } else {
                         cvr_coef<T, D> cf{ cb };
                         if constexpr (DFD)
                             cvr_update_df<D>(R[j], Rl[j], e, P[j], cf);
                         else
-                            cvr_update<T, D>(R[j], e, P[j], cf);
+                            cvr_update(R[j], e, P[j], cf);
                     }
                 } else if constexpr (DFD) {
                     cayley_update_df<LEV>(R[j], Rl[j], e, P[j], cb);
