@@ -546,7 +546,7 @@ struct dbuf {
 
 static const uint64_t GUARD_FRONT = 512;  // >= largest halo
 static const uint64_t GUARD_BACK = 8192;  // >= widest tile
-static const int MAX_DEPTH = 256;
+static const int MAX_DEPTH = 256;  // = TILE_MAX_STEPS of the kernels
 
 static std::mutex g_tune_mutex;
 static std::map<std::string, tuning> g_tune_cache;

@@ -245,8 +245,9 @@ __device__ __forceinline__ void tile_steps_pair(
         // ---- recording (solver_cpu_fdtd.tpp:288-325)
         if (p.record) {
             for (int r = 0; r < nrec; r++) {
+                if (!tl.overflow && !tl.is_due(r, m)) continue;
                 const rec_desc rc = tl.overflow ? p.recs[rd.rec_begin + r] : tl.rec[r];
-                if (rc.ratio != 1.0 && !hasto_record(rc.ratio, n)) continue;
+                if (tl.overflow && rc.ratio != 1.0 && !hasto_record(rc.ratio, n)) continue;
                 const int64_t lo = max((int64_t) rc.pos, (int64_t) td.out_start);
                 const int64_t hi = min((int64_t) rc.pos + rc.cols, (int64_t) td.out_start + td.out_len);
                 if (l0 + C <= lo || l0 >= hi) continue;
