@@ -433,8 +433,8 @@ int mbg_material_constants(
             cudaFree(dcode);
         } else {
             std::vector<double> ws(ws_n);
-            code = kind == mbg::ALGO_CVR ? mbg::pre::cvr_precompute(in, N, ws.data(), res.data())
-                                         : mbg::pre::cay_precompute(in, N, ws.data(), res.data());
+            code = kind == mbg::ALGO_CVR ? mbg::pre::cvr_precompute(in, N, ws.data(), res.data(), mbg::pre::serial_group())
+                                         : mbg::pre::cay_precompute(in, N, ws.data(), res.data(), mbg::pre::serial_group());
         }
         if (code == 1) throw mbg::invalid_argument("Number of energy levels does not match selected solver!");
         if (code == 2) throw mbg::invalid_argument("Time-indepent matrix not invertible!");

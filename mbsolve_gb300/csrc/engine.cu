@@ -307,6 +307,8 @@ run_setup setup_run(const solver_kind& k, const mbg_device* dev, const mbg_scena
 
 // ------------------------------------------------------- set-up kernels
 
+// G: serial_group (one thread per material) or block_group (one CTA)
+template<class G>
 __global__ void precompute_kernel(
     const pre::mat_in* in,
     int n,
@@ -318,16 +320,29 @@ __global__ void precompute_kernel(
     int stride,
     int* codes)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    const G g;
+    const int i = g.size > 1 ? (int) blockIdx.x : (int) (blockIdx.x * blockDim.x + threadIdx.x);
+    if (i >= n) return;  // the same in all threads of a block_group
     int rc = 0;
     if (algo == ALGO_CVR)
-        rc = pre::cvr_precompute(in[i], N, ws + (size_t) i * ws_stride, out + (size_t) i * stride);
+        rc = pre::cvr_precompute(in[i], N, ws + (size_t) i * ws_stride, out + (size_t) i * stride, g);
     else if (algo == ALGO_CAYLEY)
-        rc = pre::cay_precompute(in[i], N, ws + (size_t) i * ws_stride, out + (size_t) i * stride);
-    else
+        rc = pre::cay_precompute(in[i], N, ws + (size_t) i * ws_stride, out + (size_t) i * stride, g);
+    else if (g.rank == 0)
         rc = pre::noop_precompute(in[i], out + (size_t) i * stride);
-    codes[i] = rc;
+    if (g.rank == 0) codes[i] = rc;
+}
+
+// One CTA or one thread per material. A thread's FP64 instruction costs the
+// same 64 cycles as a warp's, so one thread takes 434 ms for a 6-level
+// material (the eigen-decomposition of the 35 x 35 dipole Liouvillian most
+// of it), the same for up to thousands side by side. A CTA of four warps
+// (one per FP64 unit) shares the matrix loops: 19 ms for 128 of them. It
+// loses where materials are small (2 levels: 3 x 3 loops) or so many that
+// the chip is full of them anyway.
+bool block_precompute(int algo, int N, int n)
+{
+    return algo != ALGO_NOOP && N >= 3 && n <= 2048;
 }
 
 void launch_precompute(
@@ -342,7 +357,12 @@ void launch_precompute(
     int* codes,
     cudaStream_t s)
 {
-    precompute_kernel<<<(unsigned) ((n + 63) / 64), 64, 0, s>>>(in, n, algo, N, ws, ws_stride, out, stride, codes);
+    if (block_precompute(algo, N, n))
+        precompute_kernel<pre::block_group>
+            <<<(unsigned) n, 128, 0, s>>>(in, n, algo, N, ws, ws_stride, out, stride, codes);
+    else
+        precompute_kernel<pre::serial_group>
+            <<<(unsigned) ((n + 63) / 64), 64, 0, s>>>(in, n, algo, N, ws, ws_stride, out, stride, codes);
 }
 
 template<typename T>
@@ -969,7 +989,7 @@ private:
         MBG_CK(cudaMemsetAsync(step_.p, 0, sizeof(unsigned long long), stream_));
         MBG_CK(cudaMemsetAsync(step_zero_.p, 0, sizeof(unsigned long long), stream_));
 
-        // materials: FP64 precompute on the GPU, one thread per material
+        // materials: FP64 precompute on the GPU
         std::vector<pre::mat_in> mins;
         std::vector<uint32_t> mat_base;
         for (const auto& r : runs_) {
@@ -1002,8 +1022,8 @@ private:
             mc64_.alloc(nm * mstride_);
             MBG_CK(cudaMemcpyAsync(din.p, mins.data(), mins.size() * sizeof(pre::mat_in),
                                    cudaMemcpyHostToDevice, stream_));
-            precompute_kernel<<<(unsigned) ((mins.size() + 63) / 64), 64, 0, stream_>>>(
-                din.p, (int) mins.size(), kind_.algo, N, ws.p, ws_stride, mc64_.p, mstride_, codes.p);
+            launch_precompute(din.p, (int) mins.size(), kind_.algo, N, ws.p, ws_stride, mc64_.p, mstride_, codes.p,
+                              stream_);
             MBG_CK(cudaGetLastError());
             std::vector<int> hc(mins.size());
             MBG_CK(cudaMemcpyAsync(hc.data(), codes.p, hc.size() * sizeof(int),

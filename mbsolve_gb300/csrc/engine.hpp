@@ -112,7 +112,9 @@ std::unique_ptr<engine> make_engine(
     std::vector<run_setup>&& runs,
     const mbg_tuning* t);
 
-// FP64 precompute of n materials on the GPU (one thread per material).
+// FP64 precompute of n materials on the GPU; block_precompute: by one CTA
+// per material (128 threads) instead of one thread.
+bool block_precompute(int algo, int N, int n);
 void launch_precompute(
     const pre::mat_in* in,
     int n,

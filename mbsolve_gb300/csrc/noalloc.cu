@@ -30,6 +30,9 @@ constexpr size_t NOALLOC_STATUS_SLOT = NOALLOC_WS_DOUBLES - 1;
 
 static __device__ __align__(256) double g_noalloc_ws[NOALLOC_WS_DOUBLES];
 
+// one CTA, or one thread where a material's matrices are small
+// (block_precompute)
+template<class G>
 __global__ void precompute_noalloc_kernel(
     const mbg::pre::mat_in m,
     int algo,
@@ -37,15 +40,15 @@ __global__ void precompute_noalloc_kernel(
     double* ws,
     double* out)
 {
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
+    const G g;
     int* code = reinterpret_cast<int*>(ws + NOALLOC_STATUS_SLOT);
-    *code = -1;  // cleared first: the slot holds the previous call's value
+    if (g.rank == 0) *code = -1;  // cleared first: the slot holds the previous call's value
     int rc;
     if (algo == mbg::ALGO_CVR)
-        rc = mbg::pre::cvr_precompute(m, N, ws, out);
+        rc = mbg::pre::cvr_precompute(m, N, ws, out, g);
     else
-        rc = mbg::pre::cay_precompute(m, N, ws, out);
-    *code = rc;
+        rc = mbg::pre::cay_precompute(m, N, ws, out, g);
+    if (g.rank == 0) *code = rc;
 }
 
 // Device address of g_noalloc_ws on the current device. The host-side
@@ -149,7 +152,10 @@ int mbg_material_constants_noalloc(
             throw mbg::invalid_argument("Unsupported superoperator!");
         double* ws = noalloc_workspace();
         cudaStream_t s = static_cast<cudaStream_t>(stream);
-        precompute_noalloc_kernel<<<1, 1, 0, s>>>(in, kind, N, ws, out_device);
+        if (mbg::block_precompute(kind, N, 1))
+            precompute_noalloc_kernel<mbg::pre::block_group><<<1, 128, 0, s>>>(in, kind, N, ws, out_device);
+        else
+            precompute_noalloc_kernel<mbg::pre::serial_group><<<1, 1, 0, s>>>(in, kind, N, ws, out_device);
         MBG_CK(cudaGetLastError());
         int code = 0;
         MBG_CK(cudaMemcpyAsync(&code, ws + NOALLOC_STATUS_SLOT, sizeof(int), cudaMemcpyDeviceToHost, s));

@@ -1,7 +1,8 @@
 // FP64 precompute of the per-material constants the time-step kernels use.
 //
 // One code path for host and device (__host__ __device__): the solvers run
-// it on the GPU, one thread per material; tests without a GPU run the host
+// it on the GPU, one thread or one CTA per material (block_precompute in
+// engine.cu); tests without a GPU run the host
 // instantiation through mbg_material_constants().
 //
 // Coherence-vector / Rodrigues form (algo_lindblad_cvr_rodr.hpp:143-229,
@@ -263,45 +264,87 @@ MBG_HD cay_layout make_cay_layout(int N)
 // column-major order: (0,1), (0,2), (1,2), (0,3), ...
 MBG_HD int upper_index(int j, int k) { return k * (k - 1) / 2 + j; }
 
+// -------------------------------------------------------------- groups
+//
+// The threads that work on one material. Loops over independent entries are
+// strided over the group; every entry is computed by one thread in the
+// serial order, sums are not split, and what every thread needs (pivots,
+// norms, rotation angles) each computes for itself, so that the results are
+// those of one thread. sync() stands between a write and another thread's
+// read of it, and between a read and another thread's overwriting.
+
+struct serial_group {
+    static constexpr int rank = 0, size = 1;
+    MBG_HD void sync() const {}
+};
+
+// the threads of a CTA (device only)
+struct block_group {
+    int rank, size;
+    MBG_HD block_group()
+    {
+#ifdef __CUDA_ARCH__
+        rank = (int) threadIdx.x;
+        size = (int) blockDim.x;
+#else
+        rank = 0;
+        size = 1;
+#endif
+    }
+    MBG_HD void sync() const
+    {
+#ifdef __CUDA_ARCH__
+        __syncthreads();
+#endif
+    }
+};
+
 // --------------------------------------------------------- small linalg
 
 // C = A * B, n x n row-major
-MBG_HD void mat_mul(const double* A, const double* B, double* C, int n)
+template<class G>
+MBG_HD void mat_mul(const double* A, const double* B, double* C, int n, const G& g)
 {
-    for (int i = 0; i < n; i++)
-        for (int j = 0; j < n; j++) {
-            double s = 0.0;
-            for (int k = 0; k < n; k++) s += A[i * n + k] * B[k * n + j];
-            C[i * n + j] = s;
-        }
+    for (int e = g.rank; e < n * n; e += g.size) {
+        const int i = e / n, j = e % n;
+        double s = 0.0;
+        for (int k = 0; k < n; k++) s += A[i * n + k] * B[k * n + j];
+        C[e] = s;
+    }
 }
 
-MBG_HD double norm1(const double* A, int n)
+// largest column sum; ws: n doubles
+template<class G>
+MBG_HD double norm1(const double* A, int n, double* ws, const G& g)
 {
-    double m = 0.0;
-    for (int j = 0; j < n; j++) {
+    for (int j = g.rank; j < n; j += g.size) {
         double s = 0.0;
         for (int i = 0; i < n; i++) s += fabs(A[i * n + j]);
-        m = s > m ? s : m;
+        ws[j] = s;
     }
+    g.sync();
+    double m = 0.0;
+    for (int j = 0; j < n; j++) m = ws[j] > m ? ws[j] : m;
+    g.sync();
     return m;
 }
 
 // F = exp(X) - I by scaling and squaring of a truncated Taylor series.
 // ws: 3 n^2 doubles.
-MBG_HD void expm_minus_identity(const double* X, double* F, int n, double* ws)
+template<class G>
+MBG_HD void expm_minus_identity(const double* X, double* F, int n, double* ws, const G& g)
 {
     double* Y = ws;
     double* T = ws + n * n;
     double* W = ws + 2 * n * n;
-    double nrm = norm1(X, n);
+    double nrm = norm1(X, n, W, g);
     int s = 0;
     while (nrm > 0.25 && s < 200) {
         nrm *= 0.5;
         s++;
     }
     double scale = ldexp(1.0, -s);
-    for (int i = 0; i < n * n; i++) Y[i] = X[i] * scale;
+    for (int i = g.rank; i < n * n; i += g.size) Y[i] = X[i] * scale;
     // degree: smallest m with nrm^(m+1)/(m+1)! below 2^-60
     int m = 1;
     double term = nrm;
@@ -310,140 +353,166 @@ MBG_HD void expm_minus_identity(const double* X, double* F, int n, double* ws)
         if (term < 8.7e-19) break;
         m++;
     }
-    // F = Y (I + Y/2 (I + Y/3 (... (I + Y/m))))  (Horner form of e^Y - I)
-    for (int i = 0; i < n * n; i++) T[i] = 0.0;
+    // F = Y (I + Y/2 (I + Y/3 (... (I + Y/m))))  (Horner form of e^Y - I);
+    // T holds the bracket with its identity
+    for (int i = g.rank; i < n * n; i += g.size) T[i] = (i % (n + 1) == 0) ? 1.0 : 0.0;
+    g.sync();
     for (int k = m; k >= 1; k--) {
-        // T <- Y (I + T) / k   (T holds the bracket without its identity)
-        for (int i = 0; i < n; i++) T[i * n + i] += 1.0;
-        mat_mul(Y, T, W, n);
-        for (int i = 0; i < n * n; i++) T[i] = W[i] / k;
+        mat_mul(Y, T, W, n, g);
+        g.sync();
+        // T <- Y T / k (+ I for the next bracket)
+        for (int i = g.rank; i < n * n; i += g.size) {
+            T[i] = W[i] / k;
+            if (k > 1 && i % (n + 1) == 0) T[i] += 1.0;
+        }
+        g.sync();
     }
-    for (int i = 0; i < n * n; i++) F[i] = T[i];
+    for (int i = g.rank; i < n * n; i += g.size) F[i] = T[i];
     // squaring: e^{2Y} - I = F (F + 2 I)
     for (int q = 0; q < s; q++) {
-        for (int i = 0; i < n * n; i++) T[i] = F[i];
-        for (int i = 0; i < n; i++) T[i * n + i] += 2.0;
-        mat_mul(F, T, W, n);
-        for (int i = 0; i < n * n; i++) F[i] = W[i];
+        for (int i = g.rank; i < n * n; i += g.size) T[i] = (i % (n + 1) == 0) ? F[i] + 2.0 : F[i];
+        g.sync();
+        mat_mul(F, T, W, n, g);
+        g.sync();
+        for (int i = g.rank; i < n * n; i += g.size) F[i] = W[i];
     }
+    g.sync();
 }
 
 // Solve A x = b by Gaussian elimination with partial pivoting (A, b are
 // overwritten). Returns 0, or 1 if a pivot is exactly zero.
-MBG_HD int solve_partial_pivot(double* A, double* b, double* x, int n)
+template<class G>
+MBG_HD int solve_partial_pivot(double* A, double* b, double* x, int n, const G& g)
 {
     int singular = 0;
     for (int k = 0; k < n; k++) {
         int p = k;
         for (int i = k + 1; i < n; i++)
             if (fabs(A[i * n + k]) > fabs(A[p * n + k])) p = i;
+        g.sync();
         if (p != k) {
-            for (int j = 0; j < n; j++) {
+            for (int j = g.rank; j < n; j += g.size) {
                 double t = A[k * n + j];
                 A[k * n + j] = A[p * n + j];
                 A[p * n + j] = t;
             }
-            double t = b[k];
-            b[k] = b[p];
-            b[p] = t;
+            if (g.rank == 0) {
+                double t = b[k];
+                b[k] = b[p];
+                b[p] = t;
+            }
         }
+        g.sync();
         double piv = A[k * n + k];
         if (piv == 0.0) {
             singular = 1;
             continue;
         }
-        for (int i = k + 1; i < n; i++) {
+        for (int i = k + 1 + g.rank; i < n; i += g.size) {
             double f = A[i * n + k] / piv;
             for (int j = k; j < n; j++) A[i * n + j] -= f * A[k * n + j];
             b[i] -= f * b[k];
         }
+        g.sync();
     }
-    for (int k = n - 1; k >= 0; k--) {
-        double piv = A[k * n + k];
-        if (piv == 0.0) {
-            x[k] = 0.0;
-            continue;
+    if (g.rank == 0)
+        for (int k = n - 1; k >= 0; k--) {
+            double piv = A[k * n + k];
+            if (piv == 0.0) {
+                x[k] = 0.0;
+                continue;
+            }
+            double s = b[k];
+            for (int j = k + 1; j < n; j++) s -= A[k * n + j] * x[j];
+            x[k] = s / piv;
         }
-        double s = b[k];
-        for (int j = k + 1; j < n; j++) s -= A[k * n + j] * x[j];
-        x[k] = s / piv;
-    }
+    g.sync();
     return singular;
 }
 
 // Cyclic Jacobi eigen-decomposition of a complex Hermitian n x n matrix
 // (re/im row-major, overwritten; the diagonal ends as the eigenvalues).
-// Eigenvectors are the columns of (vre, vim).
+// Eigenvectors are the columns of (vre, vim). ws: 2 n doubles.
+template<class G>
 MBG_HD void jacobi_hermitian(
     double* are,
     double* aim,
     double* vre,
     double* vim,
-    int n)
+    int n,
+    double* ws,
+    const G& g)
 {
-    for (int i = 0; i < n * n; i++) {
+    for (int i = g.rank; i < n * n; i += g.size) {
         vre[i] = (i % (n + 1) == 0) ? 1.0 : 0.0;
         vim[i] = 0.0;
     }
+    g.sync();
     for (int sweep = 0; sweep < 60; sweep++) {
-        double off = 0.0, tot = 0.0;
-        for (int i = 0; i < n; i++)
+        // row sums of |a|^2, all and off-diagonal
+        for (int i = g.rank; i < n; i += g.size) {
+            double off = 0.0, tot = 0.0;
             for (int j = 0; j < n; j++) {
                 double m2 = are[i * n + j] * are[i * n + j] +
                     aim[i * n + j] * aim[i * n + j];
                 tot += m2;
                 if (i != j) off += m2;
             }
+            ws[i] = off;
+            ws[n + i] = tot;
+        }
+        g.sync();
+        double off = 0.0, tot = 0.0;
+        for (int i = 0; i < n; i++) {
+            off += ws[i];
+            tot += ws[n + i];
+        }
+        g.sync();
         if (off <= 1e-32 * tot) break;
         for (int p = 0; p < n - 1; p++)
             for (int q = p + 1; q < n; q++) {
                 double zr = are[p * n + q], zi = aim[p * n + q];
+                double app = are[p * n + p], aqq = are[q * n + q];
                 double r = sqrt(zr * zr + zi * zi);
                 if (r == 0.0) continue;
                 double ephr = zr / r, ephi = zi / r;  // e^{i phi}
-                double app = are[p * n + p], aqq = are[q * n + q];
                 double tau = (aqq - app) / (2.0 * r);
                 double t = (tau >= 0 ? 1.0 : -1.0) /
                     (fabs(tau) + sqrt(1.0 + tau * tau));
                 double c = 1.0 / sqrt(1.0 + t * t), s = t * c;
+                g.sync();
                 // J = [[c, s], [-s e^{-i phi}, c e^{-i phi}]] on (p, q)
-                // columns: X <- X J
-                for (int k = 0; k < n; k++) {
-                    double xpr = are[k * n + p], xpi = aim[k * n + p];
-                    double xqr = are[k * n + q], xqi = aim[k * n + q];
+                // columns: X <- X J, of the matrix (entry e < n) and of the
+                // eigenvectors (row e - n; always the same thread's)
+                for (int e = g.rank; e < 2 * n; e += g.size) {
+                    double* re = e < n ? are + e * n : vre + (e - n) * n;
+                    double* im = e < n ? aim + e * n : vim + (e - n) * n;
+                    double xpr = re[p], xpi = im[p];
+                    double xqr = re[q], xqi = im[q];
                     // e^{-i phi} x_q
                     double yr = ephr * xqr + ephi * xqi;
                     double yi = ephr * xqi - ephi * xqr;
-                    are[k * n + p] = c * xpr - s * yr;
-                    aim[k * n + p] = c * xpi - s * yi;
-                    are[k * n + q] = s * xpr + c * yr;
-                    aim[k * n + q] = s * xpi + c * yi;
+                    re[p] = c * xpr - s * yr;
+                    im[p] = c * xpi - s * yi;
+                    re[q] = s * xpr + c * yr;
+                    im[q] = s * xpi + c * yi;
                 }
+                g.sync();
                 // rows: X <- J^H X
-                for (int k = 0; k < n; k++) {
+                for (int k = g.rank; k < n; k += g.size) {
                     double xpr = are[p * n + k], xpi = aim[p * n + k];
                     double xqr = are[q * n + k], xqi = aim[q * n + k];
                     // e^{+i phi} x_q
                     double yr = ephr * xqr - ephi * xqi;
                     double yi = ephr * xqi + ephi * xqr;
-                    are[p * n + k] = c * xpr - s * yr;
-                    aim[p * n + k] = c * xpi - s * yi;
-                    are[q * n + k] = s * xpr + c * yr;
-                    aim[q * n + k] = s * xpi + c * yi;
+                    // the pair's off-diagonal entries vanish, the diagonal
+                    // ones are real
+                    are[p * n + k] = k == q ? 0.0 : c * xpr - s * yr;
+                    aim[p * n + k] = k == q || k == p ? 0.0 : c * xpi - s * yi;
+                    are[q * n + k] = k == p ? 0.0 : s * xpr + c * yr;
+                    aim[q * n + k] = k == q || k == p ? 0.0 : s * xpi + c * yi;
                 }
-                are[p * n + q] = aim[p * n + q] = 0.0;
-                are[q * n + p] = aim[q * n + p] = 0.0;
-                aim[p * n + p] = aim[q * n + q] = 0.0;
-                for (int k = 0; k < n; k++) {
-                    double xpr = vre[k * n + p], xpi = vim[k * n + p];
-                    double xqr = vre[k * n + q], xqi = vim[k * n + q];
-                    double yr = ephr * xqr + ephi * xqi;
-                    double yi = ephr * xqi - ephi * xqr;
-                    vre[k * n + p] = c * xpr - s * yr;
-                    vim[k * n + p] = c * xpi - s * yi;
-                    vre[k * n + q] = s * xpr + c * yr;
-                    vim[k * n + q] = s * xpi + c * yi;
-                }
+                g.sync();
             }
     }
 }
@@ -612,21 +681,22 @@ MBG_HD void write_fdtd(const mat_in& m, double* out)
 // `Nsolver` levels). Returns 0 on success, 1 when the level count does not
 // match the solver, 2 when M d_in = d_eq has no solution (the reference's
 // "Time-indepent matrix not invertible!" check, rodr.hpp:195-206).
-MBG_HD int cvr_precompute(const mat_in& m, int Nsolver, double* ws, double* out)
+template<class G>
+MBG_HD int cvr_precompute(const mat_in& m, int Nsolver, double* ws, double* out, const G& g)
 {
     cvr_layout L = make_cvr_layout(Nsolver);
-    for (int i = 0; i < L.stride; i++) out[i] = 0.0;
-    write_fdtd(m, out);
+    for (int i = g.rank; i < L.stride; i += g.size) out[i] = 0.0;
+    g.sync();
+    if (g.rank == 0) write_fdtd(m, out);
     const int N = Nsolver, V = L.V, KP = L.KP;
     if (m.N == 0) {
         // no quantum-mechanical description: the density stays the zero
         // vector, whose populations are 1/N (cvr.hpp:289-336)
-        out[L.has_qm] = 0.0;
-        for (int k = 0; k < N; k++) out[L.pop_c + k] = population_const(N, k);
+        for (int k = g.rank; k < N; k += g.size) out[L.pop_c + k] = population_const(N, k);
         return 0;
     }
     if (m.N != Nsolver) return 1;
-    out[L.has_qm] = 1.0;
+    if (g.rank == 0) out[L.has_qm] = 1.0;
     const int NN = N * N;
     double* X = ws;                        // V * N*N * 2 : op * g_i
     double* Tr = X + (size_t) V * NN * 2;  // V*V*2 : tr(op g_i g_j)
@@ -647,10 +717,6 @@ MBG_HD int cvr_precompute(const mat_in& m, int Nsolver, double* ws, double* out)
     double* t2 = vec + 4 * V;
     double* lam = vec + 5 * V;
     double* d0 = vec + 6 * V;
-    double* tre = vec + 7 * V;  // N*N (<= V+1)
-    double* tim = tre + NN;
-    double* ure = tim + NN;
-    double* uim = ure + NN;
 
     int gr[8], gc[8];
     cd gv[8];
@@ -659,7 +725,7 @@ MBG_HD int cvr_precompute(const mat_in& m, int Nsolver, double* ws, double* out)
     for (int which = 0; which < 2; which++) {
         const double* ore = which == 0 ? m.h_re : m.mu_re;
         const double* oim = which == 0 ? m.h_im : m.mu_im;
-        for (int i = 0; i < V; i++) {
+        for (int i = g.rank; i < V; i += g.size) {
             int nz = generator_entries(N, i, gr, gc, gv);
             double* xr = X + (size_t) i * NN * 2;
             double* xi = xr + NN;
@@ -673,26 +739,28 @@ MBG_HD int cvr_precompute(const mat_in& m, int Nsolver, double* ws, double* out)
                     xi[rr * N + gc[e]] += p.im;
                 }
         }
-        for (int i = 0; i < V; i++)
-            for (int j = 0; j < V; j++) {
-                int nz = generator_entries(N, j, gr, gc, gv);
-                const double* xr = X + (size_t) i * NN * 2;
-                cd t = trace_with_gen(xr, xr + NN, N, nz, gr, gc, gv);
-                Tr[(i * V + j) * 2] = t.re;
-                Tr[(i * V + j) * 2 + 1] = t.im;
-            }
-        for (int i = 0; i < V; i++)
-            for (int j = 0; j < V; j++) {
-                double dim = Tr[(i * V + j) * 2 + 1] - Tr[(j * V + i) * 2 + 1];
-                double l = -0.5 * dim / HBAR;  // Re(i z / 2) = -Im(z) / 2
-                if (which == 0)
-                    M[i * V + j] = l;
-                else
-                    U[i * V + j] = -l;  // U = -L(mu)
-            }
+        g.sync();
+        for (int e = g.rank; e < V * V; e += g.size) {
+            int nz = generator_entries(N, e % V, gr, gc, gv);
+            const double* xr = X + (size_t) (e / V) * NN * 2;
+            cd t = trace_with_gen(xr, xr + NN, N, nz, gr, gc, gv);
+            Tr[e * 2] = t.re;
+            Tr[e * 2 + 1] = t.im;
+        }
+        g.sync();
+        for (int e = g.rank; e < V * V; e += g.size) {
+            const int i = e / V, j = e % V;
+            double dim = Tr[(i * V + j) * 2 + 1] - Tr[(j * V + i) * 2 + 1];
+            double l = -0.5 * dim / HBAR;  // Re(i z / 2) = -Im(z) / 2
+            if (which == 0)
+                M[e] = l;
+            else
+                U[e] = -l;  // U = -L(mu)
+        }
+        g.sync();
         if (which == 1) {
             // dipole vector v_i = Re tr(mu g_i) (cvr.hpp:168-179)
-            for (int i = 0; i < V; i++) {
+            for (int i = g.rank; i < V; i += g.size) {
                 int nz = generator_entries(N, i, gr, gc, gv);
                 v_dip[i] = trace_with_gen(m.mu_re, m.mu_im, N, nz, gr, gc, gv).re;
             }
@@ -700,7 +768,8 @@ MBG_HD int cvr_precompute(const mat_in& m, int Nsolver, double* ws, double* out)
     }
     // relaxation superoperator G_ij = Re 1/2 tr(R(g_j) g_i) and the
     // equilibrium vector d_eq_i = Re tr(R(I) g_i) / N (cvr.hpp:181-213)
-    for (int j = 0; j < V; j++) {
+    double tre[36], tim[36], ure[36], uim[36];
+    for (int j = g.rank; j < V; j += g.size) {
         int nz = generator_entries(N, j, gr, gc, gv);
         for (int e = 0; e < NN; e++) tre[e] = tim[e] = 0.0;
         for (int e = 0; e < nz; e++) {
@@ -719,10 +788,11 @@ MBG_HD int cvr_precompute(const mat_in& m, int Nsolver, double* ws, double* out)
         tim[e] = 0.0;
     }
     relax_apply(m, tre, tim, ure, uim);
-    for (int i = 0; i < V; i++) {
+    for (int i = g.rank; i < V; i += g.size) {
         int nz = generator_entries(N, i, gr, gc, gv);
         d_eq[i] = trace_with_gen(ure, uim, N, nz, gr, gc, gv).re / N;
     }
+    g.sync();
     const double M_CP = 0.5 * m.carrier_density;
 
     // d_in: M d_in = d_eq unless d_eq is zero (rodr.hpp:193-206)
@@ -730,32 +800,42 @@ MBG_HD int cvr_precompute(const mat_in& m, int Nsolver, double* ws, double* out)
     for (int i = 0; i < V; i++)
         if (fabs(d_eq[i]) > 2.220446049250313e-16) zero = false;
     if (zero) {
-        for (int i = 0; i < V; i++) d_in[i] = 0.0;
+        for (int i = g.rank; i < V; i += g.size) d_in[i] = 0.0;
+        g.sync();
     } else {
-        for (int i = 0; i < V * V; i++) F[i] = M[i];
-        for (int i = 0; i < V; i++) t1[i] = d_eq[i];
-        solve_partial_pivot(F, t1, d_in, V);
-        double nr = 0.0, nd = 0.0;
-        for (int i = 0; i < V; i++) {
+        for (int i = g.rank; i < V * V; i += g.size) F[i] = M[i];
+        for (int i = g.rank; i < V; i += g.size) t1[i] = d_eq[i];
+        g.sync();
+        solve_partial_pivot(F, t1, d_in, V, g);
+        for (int i = g.rank; i < V; i += g.size) {
             double s = -d_eq[i];
             for (int j = 0; j < V; j++) s += M[i * V + j] * d_in[j];
-            nr += s * s;
+            t2[i] = s;
+        }
+        g.sync();
+        double nr = 0.0, nd = 0.0;
+        for (int i = 0; i < V; i++) {
+            nr += t2[i] * t2[i];
             nd += d_eq[i] * d_eq[i];
         }
+        g.sync();
         if (!(sqrt(nr) / sqrt(nd) <= 1e-3)) return 2;
     }
 
     // F = exp(M dt/2) - I
-    for (int i = 0; i < V * V; i++) H1[i] = M[i] * m.dt / 2;
-    expm_minus_identity(H1, F, V, W);
+    for (int i = g.rank; i < V * V; i += g.size) H1[i] = M[i] * m.dt / 2;
+    g.sync();
+    expm_minus_identity(H1, F, V, W, g);
 
     // planes of U from the Hermitian matrix i U
-    for (int i = 0; i < V * V; i++) {
+    for (int i = g.rank; i < V * V; i += g.size) {
         H1[i] = 0.0;
         H2[i] = U[i];
     }
-    jacobi_hermitian(H1, H2, E1, E2, V);
-    for (int i = 0; i < V; i++) lam[i] = H1[i * V + i];
+    g.sync();
+    jacobi_hermitian(H1, H2, E1, E2, V, W, g);
+    for (int i = g.rank; i < V; i += g.size) lam[i] = H1[i * V + i];
+    g.sync();
     double lmax = 0.0;
     for (int i = 0; i < V; i++) lmax = lam[i] > lmax ? lam[i] : lmax;
     int used[64];
@@ -771,10 +851,12 @@ MBG_HD int cvr_precompute(const mat_in& m, int Nsolver, double* ws, double* out)
         used[best] = 1;
         // q1, q2 from the real and imaginary parts, re-orthonormalised
         double n1 = 0.0;
-        for (int i = 0; i < V; i++) {
+        g.sync();
+        for (int i = g.rank; i < V; i += g.size) {
             t1[i] = E1[i * V + best];
             t2[i] = E2[i * V + best];
         }
+        g.sync();
         for (int pass = 0; pass < 2; pass++)
             for (int col = 0; col < ncol; col++) {
                 double d1 = 0.0, d2 = 0.0;
@@ -782,100 +864,111 @@ MBG_HD int cvr_precompute(const mat_in& m, int Nsolver, double* ws, double* out)
                     d1 += Q[i * V + col] * t1[i];
                     d2 += Q[i * V + col] * t2[i];
                 }
-                for (int i = 0; i < V; i++) {
+                g.sync();
+                for (int i = g.rank; i < V; i += g.size) {
                     t1[i] -= d1 * Q[i * V + col];
                     t2[i] -= d2 * Q[i * V + col];
                 }
+                g.sync();
             }
         for (int i = 0; i < V; i++) n1 += t1[i] * t1[i];
         n1 = sqrt(n1);
         if (n1 < 1e-3) continue;
-        for (int i = 0; i < V; i++) t1[i] /= n1;
+        g.sync();
+        for (int i = g.rank; i < V; i += g.size) t1[i] /= n1;
+        g.sync();
         double dd = 0.0;
         for (int i = 0; i < V; i++) dd += t1[i] * t2[i];
+        g.sync();
+        for (int i = g.rank; i < V; i += g.size) t2[i] -= dd * t1[i];
+        g.sync();
         double n2 = 0.0;
-        for (int i = 0; i < V; i++) {
-            t2[i] -= dd * t1[i];
-            n2 += t2[i] * t2[i];
-        }
+        for (int i = 0; i < V; i++) n2 += t2[i] * t2[i];
         n2 = sqrt(n2);
         if (n2 < 1e-3) continue;
-        for (int i = 0; i < V; i++) t2[i] /= n2;
+        g.sync();
+        for (int i = g.rank; i < V; i += g.size) t2[i] /= n2;
         // theta = q2 . U q1 ; orient so that theta > 0
-        double th = 0.0;
-        for (int i = 0; i < V; i++) {
+        for (int i = g.rank; i < V; i += g.size) {
             double s = 0.0;
             for (int j = 0; j < V; j++) s += U[i * V + j] * t1[j];
-            th += t2[i] * s;
+            W[i] = s;
         }
-        if (th < 0) {
-            th = -th;
-            for (int i = 0; i < V; i++) t2[i] = -t2[i];
-        }
-        for (int i = 0; i < V; i++) {
+        g.sync();
+        double th = 0.0;
+        for (int i = 0; i < V; i++) th += t2[i] * W[i];
+        const double sign = th < 0 ? -1.0 : 1.0;
+        for (int i = g.rank; i < V; i += g.size) {
             Q[i * V + ncol] = t1[i];
-            Q[i * V + ncol + 1] = t2[i];
+            Q[i * V + ncol + 1] = sign * t2[i];
         }
-        out[L.thdt + nplanes] = th * m.dt;
+        if (g.rank == 0) out[L.thdt + nplanes] = sign * th * m.dt;
+        g.sync();
         ncol += 2;
         nplanes++;
     }
-    out[L.nplanes] = nplanes;
+    if (g.rank == 0) out[L.nplanes] = nplanes;
     // complete Q with an orthonormal basis of the null space of U
     while (ncol < V) {
         int best = -1;
         double bestn = -1.0;
-        for (int i = 0; i < V; i++) {
+        for (int i = g.rank; i < V; i += g.size) {
             double s = 1.0;
             for (int col = 0; col < ncol; col++)
                 s -= Q[i * V + col] * Q[i * V + col];
-            if (s > bestn) {
-                bestn = s;
+            W[i] = s;
+        }
+        g.sync();
+        for (int i = 0; i < V; i++)
+            if (W[i] > bestn) {
+                bestn = W[i];
                 best = i;
             }
-        }
-        for (int i = 0; i < V; i++) t1[i] = (i == best) ? 1.0 : 0.0;
+        for (int i = g.rank; i < V; i += g.size) t1[i] = (i == best) ? 1.0 : 0.0;
+        g.sync();
         for (int pass = 0; pass < 2; pass++)
             for (int col = 0; col < ncol; col++) {
                 double d = 0.0;
                 for (int i = 0; i < V; i++) d += Q[i * V + col] * t1[i];
-                for (int i = 0; i < V; i++) t1[i] -= d * Q[i * V + col];
+                g.sync();
+                for (int i = g.rank; i < V; i += g.size) t1[i] -= d * Q[i * V + col];
+                g.sync();
             }
         double nn = 0.0;
         for (int i = 0; i < V; i++) nn += t1[i] * t1[i];
         nn = sqrt(nn);
-        for (int i = 0; i < V; i++) Q[i * V + ncol] = t1[i] / nn;
+        for (int i = g.rank; i < V; i += g.size) Q[i * V + ncol] = t1[i] / nn;
+        g.sync();
         ncol++;
     }
 
-    for (int i = 0; i < V * V; i++) out[L.Q + i] = Q[i];
+    for (int i = g.rank; i < V * V; i += g.size) out[L.Q + i] = Q[i];
     // out[o] = Q^T X Q for X (V x V, original basis); H1 is scratch
     auto to_planes = [&](const double* X, double* dst) {
-        for (int i = 0; i < V; i++)
-            for (int j = 0; j < V; j++) {
-                double s = 0.0;
-                for (int k = 0; k < V; k++) s += X[i * V + k] * Q[k * V + j];
-                H1[i * V + j] = s;  // X Q
-            }
-        for (int i = 0; i < V; i++)
-            for (int j = 0; j < V; j++) {
-                double s = 0.0;
-                for (int k = 0; k < V; k++) s += Q[k * V + i] * H1[k * V + j];
-                dst[i * V + j] = s;
-            }
+        mat_mul(X, Q, H1, V, g);
+        g.sync();
+        for (int e = g.rank; e < V * V; e += g.size) {
+            const int i = e / V, j = e % V;
+            double s = 0.0;
+            for (int k = 0; k < V; k++) s += Q[k * V + i] * H1[k * V + j];
+            dst[e] = s;
+        }
+        g.sync();
     };
     // Q^T X d_in
     auto drive = [&](const double* X, double* dst) {
-        for (int i = 0; i < V; i++) {
+        for (int i = g.rank; i < V; i += g.size) {
             double s = 0.0;
             for (int j = 0; j < V; j++) s += X[i * V + j] * d_in[j];
             t2[i] = s;
         }
-        for (int k = 0; k < V; k++) {
+        g.sync();
+        for (int k = g.rank; k < V; k += g.size) {
             double s = 0.0;
             for (int i = 0; i < V; i++) s += Q[i * V + k] * t2[i];
             dst[k] = s;
         }
+        g.sync();
     };
     // half step: Bh = Q^T (exp(M dt/2) - I) Q, kh = Q^T (exp(M dt/2) - I) d_in
     double* Bh = out + L.Bh;
@@ -883,71 +976,77 @@ MBG_HD int cvr_precompute(const mat_in& m, int Nsolver, double* ws, double* out)
     to_planes(F, Bh);
     drive(F, kh);
     // full step: Bd = Q^T (exp(M dt) - I) Q, k = Q^T (exp(M dt) - I) d_in
-    for (int i = 0; i < V * V; i++) H2[i] = M[i] * m.dt;
-    expm_minus_identity(H2, E1, V, W);
+    for (int i = g.rank; i < V * V; i += g.size) H2[i] = M[i] * m.dt;
+    g.sync();
+    expm_minus_identity(H2, E1, V, W, g);
     to_planes(E1, out + L.Bd);
-    for (int i = 0; i < V * V; i++) out[L.Bdl + i] = out[L.Bd + i] - (double) (float) out[L.Bd + i];
+    for (int i = g.rank; i < V * V; i += g.size) out[L.Bdl + i] = out[L.Bd + i] - (double) (float) out[L.Bd + i];
     drive(E1, out + L.k);
     // Bi = A^-1 - I = Q^T (exp(-M dt/2) - I) Q
-    for (int i = 0; i < V * V; i++) H2[i] = -M[i] * m.dt / 2;
-    expm_minus_identity(H2, E2, V, W);
+    for (int i = g.rank; i < V * V; i += g.size) H2[i] = -M[i] * m.dt / 2;
+    g.sync();
+    expm_minus_identity(H2, E2, V, W, g);
     double* Bi = E1;
     to_planes(E2, Bi);
-    // a row r on u becomes r (I + Bi) on v with constant -r (I + Bi) kh
-    auto compose = [&](double* r, double& c) {
-        for (int j = 0; j < V; j++) {
+    // a row r on u becomes r (I + Bi) on v with constant c - r (I + Bi) kh,
+    // stored at dst
+    auto compose = [&](double* r, double c, double* dst) {
+        g.sync();
+        for (int j = g.rank; j < V; j += g.size) {
             double s = r[j];
             for (int i = 0; i < V; i++) s += r[i] * Bi[i * V + j];
             t1[j] = s;
         }
-        for (int j = 0; j < V; j++) {
-            r[j] = t1[j];
-            c -= t1[j] * kh[j];
+        g.sync();
+        for (int j = g.rank; j < V; j += g.size) r[j] = t1[j];
+        if (g.rank == 0) {
+            for (int j = 0; j < V; j++) c -= t1[j] * kh[j];
+            *dst = c;
         }
+        g.sync();
     };
     // P = p0 + g . u with g = M_CP Q^T M^T v_dip, p0 = M_CP v_dip . d_eq
     // (rodr.hpp:258-266)
-    for (int j = 0; j < V; j++) {
+    for (int j = g.rank; j < V; j += g.size) {
         double s = 0.0;
         for (int i = 0; i < V; i++) s += M[i * V + j] * v_dip[i];
         t2[j] = s;  // (M^T v)_j
     }
+    g.sync();
     double p0 = 0.0;
     for (int i = 0; i < V; i++) p0 += v_dip[i] * d_eq[i];
-    for (int k = 0; k < V; k++) {
+    for (int k = g.rank; k < V; k += g.size) {
         double sg = 0.0;
         for (int i = 0; i < V; i++) sg += Q[i * V + k] * t2[i];
         out[L.g + k] = M_CP * sg;
     }
     p0 *= M_CP;
-    compose(out + L.g, p0);
-    out[L.p0] = p0;
+    compose(out + L.g, p0, out + L.p0);
     // initial state v0 = A u0 + kh, u0 = Q^T d0
-    initial_coherence_vector(m, d0);
-    for (int k = 0; k < V; k++) {
+    if (g.rank == 0) initial_coherence_vector(m, d0);
+    g.sync();
+    for (int k = g.rank; k < V; k += g.size) {
         double s = 0.0;
         for (int i = 0; i < V; i++) s += Q[i * V + k] * d0[i];
         t2[k] = s;
     }
-    for (int i = 0; i < V; i++) {
+    g.sync();
+    for (int i = g.rank; i < V; i += g.size) {
         double s = t2[i] + kh[i];
         for (int j = 0; j < V; j++) s += Bh[i * V + j] * t2[j];
         out[L.z0 + i] = s;
     }
     // observables: d = Q u
     int w0 = N * (N - 1);
-    for (int k = 0; k < V; k++) out[L.inv + k] = Q[w0 * V + k];
-    out[L.inv_c] = 0.0;
-    compose(out + L.inv, out[L.inv_c]);
+    for (int k = g.rank; k < V; k += g.size) out[L.inv + k] = Q[w0 * V + k];
+    compose(out + L.inv, 0.0, out + L.inv_c);
     for (int mm = 0; mm < N; mm++) {
-        for (int k = 0; k < V; k++) out[L.pop + mm * V + k] = 0.0;
-        for (int i = 0; i < N - 1; i++) {
-            double w = 0.5 * population_weight(N, mm, i);
-            for (int k = 0; k < V; k++)
-                out[L.pop + mm * V + k] += w * Q[(w0 + i) * V + k];
+        for (int k = g.rank; k < V; k += g.size) {
+            double s = 0.0;
+            for (int i = 0; i < N - 1; i++) s += 0.5 * population_weight(N, mm, i) * Q[(w0 + i) * V + k];
+            out[L.pop + mm * V + k] = s;
         }
-        out[L.pop_c + mm] = population_const(N, mm);
-        compose(out + L.pop + mm * V, out[L.pop_c + mm]);
+        compose(out + L.pop + mm * V, population_const(N, mm), out + L.pop_c + mm);
     }
     // coherences: rho = I/N + 1/2 sum_i d_i g_i, so rho[j][k] (j != k) is
     // 1/2 sum_i (g_i)[j][k] d_i: real and imaginary rows on d, then on u
@@ -956,20 +1055,20 @@ MBG_HD int cvr_precompute(const mat_in& m, int Nsolver, double* ws, double* out)
         for (int jj = 0; jj < kk; jj++) {
             const int q = kk * (kk - 1) / 2 + jj;
             for (int part = 0; part < 2; part++) {
-                for (int i = 0; i < V; i++) t2[i] = 0.0;
-                for (int i = 0; i < V; i++) {
+                for (int i = g.rank; i < V; i += g.size) {
+                    t2[i] = 0.0;
                     int nz = generator_entries(N, i, gr, gc, gv);
                     for (int e = 0; e < nz; e++)
                         if (gr[e] == jj && gc[e] == kk) t2[i] += 0.5 * (part == 0 ? gv[e].re : gv[e].im);
                 }
+                g.sync();
                 double* row = out + L.coh + (2 * q + part) * V;
-                for (int c = 0; c < V; c++) {
+                for (int c = g.rank; c < V; c += g.size) {
                     double s = 0.0;
                     for (int i = 0; i < V; i++) s += t2[i] * Q[i * V + c];
                     row[c] = s;
                 }
-                out[L.coh_c + 2 * q + part] = 0.0;
-                compose(row, out[L.coh_c + 2 * q + part]);
+                compose(row, 0.0, out + L.coh_c + 2 * q + part);
             }
         }
     return 0;
@@ -1016,13 +1115,15 @@ MBG_HD void herm_at(const double* p, int N, int j, int k, double& re, double& im
 //   Im rho_jk (j < k): -2 Re C_jk + 2 gamma_jk Im Mn_jk
 // (gamma_jk the dephasing rate of the pair, D'(rho)_jk = gamma_jk rho_jk).
 // Evaluated per material in FP64; the kernels then need N^2 FMAs per point.
-MBG_HD void cay_polarisation_weights(const cay_layout& L, double* out)
+template<class G>
+MBG_HD void cay_polarisation_weights(const cay_layout& L, double* out, const G& g)
 {
     const int N = L.N;
     const double* W = out + L.W0;
     const double* Mn = out + L.Mn;
     for (int j = 0; j < N; j++)
         for (int k = j; k < N; k++) {
+            if ((j * N + k) % g.size != g.rank) continue;
             // C_jk = sum_l Mn_jl W_lk - W_jl Mn_lk
             double cr = 0.0, ci = 0.0;
             for (int l = 0; l < N; l++) {
@@ -1098,35 +1199,40 @@ MBG_HD void csolve(cd* A, cd* B, int n, int m)
 }
 
 // Full Hermitian matrix (n x n, row-major) from its packed form, and back.
-MBG_HD void herm_unpack(const double* p, int N, cd* F)
+template<class G>
+MBG_HD void herm_unpack(const double* p, int N, cd* F, const G& g)
 {
-    for (int j = 0; j < N; j++)
-        for (int k = 0; k < N; k++) herm_at(p, N, j, k, F[j * N + k].re, F[j * N + k].im);
+    for (int e = g.rank; e < N * N; e += g.size) herm_at(p, N, e / N, e % N, F[e].re, F[e].im);
 }
-MBG_HD void herm_pack(const cd* F, int N, double* p)
+template<class G>
+MBG_HD void herm_pack(const cd* F, int N, double* p, const G& g)
 {
-    for (int i = 0; i < N; i++) p[i] = F[i * N + i].re;
-    for (int k = 1; k < N; k++)
-        for (int j = 0; j < k; j++) {
+    for (int e = g.rank; e < N * N; e += g.size) {
+        const int j = e / N, k = e % N;
+        if (j == k) {
+            p[j] = F[e].re;
+        } else if (j < k) {
             const int q = upper_index(j, k);
-            p[N + 2 * q] = F[j * N + k].re;
-            p[N + 2 * q + 1] = F[j * N + k].im;
+            p[N + 2 * q] = F[e].re;
+            p[N + 2 * q + 1] = F[e].im;
         }
+    }
 }
 
 // (D - I) r for the dissipation half step D on a packed density matrix:
 // populations by D1 - I, the coherence of pair q by D2_q - 1.
-MBG_HD void cay_dissipation_increment(const cay_layout& L, const double* out, const double* r, double* d)
+template<class G>
+MBG_HD void cay_dissipation_increment(const cay_layout& L, const double* out, const double* r, double* d, const G& g)
 {
     const int N = L.N;
-    for (int i = 0; i < N; i++) {
-        double s = 0.0;
-        for (int j = 0; j < N; j++) s += out[L.dD1 + i * N + j] * r[j];
-        d[i] = s;
-    }
-    for (int q = 0; q < L.P; q++) {
-        d[N + 2 * q] = out[L.dD2 + q] * r[N + 2 * q];
-        d[N + 2 * q + 1] = out[L.dD2 + q] * r[N + 2 * q + 1];
+    for (int i = g.rank; i < N * N; i += g.size) {
+        if (i < N) {
+            double s = 0.0;
+            for (int j = 0; j < N; j++) s += out[L.dD1 + i * N + j] * r[j];
+            d[i] = s;
+        } else {
+            d[i] = out[L.dD2 + (i - N) / 2] * r[i];
+        }
     }
 }
 
@@ -1139,7 +1245,8 @@ MBG_HD void cay_dissipation_increment(const cay_layout& L, const double* out, co
 // coherence (re, im) only with itself; blockB0 = 1 lets the kernels skip
 // the zero blocks (the same sums without exact zero terms).
 // ws: 17 N^2 doubles.
-MBG_HD void cay_free_step(const cay_layout& L, double* ws, double* out)
+template<class G>
+MBG_HD void cay_free_step(const cay_layout& L, double* ws, double* out, const G& g)
 {
     const int N = L.N, NN = N * N;
     cd* A = reinterpret_cast<cd*>(ws);  // NN
@@ -1147,73 +1254,83 @@ MBG_HD void cay_free_step(const cay_layout& L, double* ws, double* out)
     cd* X = B + 2 * NN;                  // X0 = U0 - I
     cd* K = X + NN;                      // K1, then scratch
     cd* S = K + NN;                      // sigma (full)
-    cd* G = S + NN;                      // X0 sigma
-    double* r = reinterpret_cast<double*>(G + NN);  // NN packed
+    cd* Gm = S + NN;                     // X0 sigma
+    double* r = reinterpret_cast<double*>(Gm + NN);  // NN packed
     double* t = r + NN;
     double* d = t + NN;
     // A0 = I + i K0; solve A0 [Y | Ai] = [K0 | I]
-    for (int j = 0; j < N; j++)
-        for (int k = 0; k < N; k++) {
-            double kr, ki;
-            herm_at(out + L.kH0, N, j, k, kr, ki);
-            A[j * N + k] = cmake((j == k ? 1.0 : 0.0) - ki, kr);
-            B[j * 2 * N + k] = cmake(kr, ki);
-            B[j * 2 * N + N + k] = cmake(j == k ? 1.0 : 0.0, 0.0);
-        }
-    csolve(A, B, N, 2 * N);
-    // X0 = -2i Y; U0 = I + X0
-    for (int j = 0; j < N; j++)
-        for (int k = 0; k < N; k++) {
-            const cd y = B[j * 2 * N + k];
-            X[j * N + k] = cmake(2.0 * y.im, -2.0 * y.re);
-            out[L.U0 + j * N + k] = (j == k ? 1.0 : 0.0) + X[j * N + k].re;
-            out[L.U0 + NN + j * N + k] = X[j * N + k].im;
-        }
+    for (int e = g.rank; e < NN; e += g.size) {
+        const int j = e / N, k = e % N;
+        double kr, ki;
+        herm_at(out + L.kH0, N, j, k, kr, ki);
+        A[e] = cmake((j == k ? 1.0 : 0.0) - ki, kr);
+        B[j * 2 * N + k] = cmake(kr, ki);
+        B[j * 2 * N + N + k] = cmake(j == k ? 1.0 : 0.0, 0.0);
+    }
+    g.sync();
+    if (g.rank == 0) csolve(A, B, N, 2 * N);
+    g.sync();
+    // X0 = -2i Y; U0 = I + X0; K1 = kappa mu
+    for (int e = g.rank; e < NN; e += g.size) {
+        const int j = e / N, k = e % N;
+        const cd y = B[j * 2 * N + k];
+        X[e] = cmake(2.0 * y.im, -2.0 * y.re);
+        out[L.U0 + e] = (j == k ? 1.0 : 0.0) + X[e].re;
+        out[L.U0 + NN + e] = X[e].im;
+        double kr, ki;
+        herm_at(out + L.kMu, N, j, k, kr, ki);
+        K[e] = cmake(kr, ki);
+    }
+    g.sync();
     // W = K1 A0^-1
-    for (int j = 0; j < N; j++)
-        for (int k = 0; k < N; k++) {
-            double kr, ki;
-            herm_at(out + L.kMu, N, j, k, kr, ki);
-            K[j * N + k] = cmake(kr, ki);
-        }
-    for (int j = 0; j < N; j++)
-        for (int k = 0; k < N; k++) {
-            cd s = cmake(0.0, 0.0);
-            for (int l = 0; l < N; l++) s = cadd(s, cmul(K[j * N + l], B[l * 2 * N + N + k]));
-            out[L.Wk + j * N + k] = s.re;
-            out[L.Wk + NN + j * N + k] = s.im;
-        }
+    for (int e = g.rank; e < NN; e += g.size) {
+        const int j = e / N, k = e % N;
+        cd s = cmake(0.0, 0.0);
+        for (int l = 0; l < N; l++) s = cadd(s, cmul(K[j * N + l], B[l * 2 * N + N + k]));
+        out[L.Wk + e] = s.re;
+        out[L.Wk + NN + e] = s.im;
+    }
     bool diag = true;
     for (int q = 0; q < L.P; q++)
         if (out[L.kH0 + N + 2 * q] != 0.0 || out[L.kH0 + N + 2 * q + 1] != 0.0) diag = false;
-    out[L.blockB0] = diag ? 1.0 : 0.0;
+    if (g.rank == 0) out[L.blockB0] = diag ? 1.0 : 0.0;
     // columns of B0: e_v -> (D - I) e_v + pack(Ad(U0) s - s) + (D - I) tau,
     // s = D e_v, tau = Ad(U0) s
     for (int v = 0; v < NN; v++) {
-        for (int i = 0; i < NN; i++) r[i] = (i == v) ? 1.0 : 0.0;
-        cay_dissipation_increment(L, out, r, d);  // (D - I) e_v
-        for (int i = 0; i < NN; i++) t[i] = r[i] + d[i];
-        herm_unpack(t, N, S);
+        g.sync();
+        for (int i = g.rank; i < NN; i += g.size) r[i] = (i == v) ? 1.0 : 0.0;
+        g.sync();
+        cay_dissipation_increment(L, out, r, d, g);  // (D - I) e_v
+        g.sync();
+        for (int i = g.rank; i < NN; i += g.size) t[i] = r[i] + d[i];
+        g.sync();
+        herm_unpack(t, N, S, g);
+        g.sync();
         // Ad(U0) s - s = X0 s + (X0 s)^H + X0 s X0^H
-        for (int j = 0; j < N; j++)
-            for (int k = 0; k < N; k++) {
-                cd g = cmake(0.0, 0.0);
-                for (int l = 0; l < N; l++) g = cadd(g, cmul(X[j * N + l], S[l * N + k]));
-                G[j * N + k] = g;
-            }
-        for (int j = 0; j < N; j++)
-            for (int k = 0; k < N; k++) {
-                cd h = cadd(G[j * N + k], cconj(G[k * N + j]));
-                for (int l = 0; l < N; l++) h = cadd(h, cmul(G[j * N + l], cconj(X[k * N + l])));
-                K[j * N + k] = h;
-            }
-        herm_pack(K, N, r);  // Ad(U0) s - s, packed
-        for (int i = 0; i < NN; i++) {
+        for (int e = g.rank; e < NN; e += g.size) {
+            const int j = e / N, k = e % N;
+            cd w = cmake(0.0, 0.0);
+            for (int l = 0; l < N; l++) w = cadd(w, cmul(X[j * N + l], S[l * N + k]));
+            Gm[e] = w;
+        }
+        g.sync();
+        for (int e = g.rank; e < NN; e += g.size) {
+            const int j = e / N, k = e % N;
+            cd h = cadd(Gm[j * N + k], cconj(Gm[k * N + j]));
+            for (int l = 0; l < N; l++) h = cadd(h, cmul(Gm[j * N + l], cconj(X[k * N + l])));
+            K[e] = h;
+        }
+        g.sync();
+        herm_pack(K, N, r, g);  // Ad(U0) s - s, packed
+        g.sync();
+        for (int i = g.rank; i < NN; i += g.size) {
             d[i] += r[i];       // column so far: (D - I) e_v + (Ad(U0) s - s)
             t[i] += r[i];       // tau = s + (Ad(U0) s - s)
         }
-        cay_dissipation_increment(L, out, t, r);  // (D - I) tau
-        for (int i = 0; i < NN; i++) {
+        g.sync();
+        cay_dissipation_increment(L, out, t, r, g);  // (D - I) tau
+        g.sync();
+        for (int i = g.rank; i < NN; i += g.size) {
             const double b = d[i] + r[i];
             out[L.B0 + i * L.NP + v] = b;
             out[L.B0l + i * L.NP + v] = b - (double) (float) b;
@@ -1224,46 +1341,49 @@ MBG_HD void cay_free_step(const cay_layout& L, double* ws, double* out)
 // Cayley constants of one material (cay_layout of `Nsolver` levels).
 // Returns 0, 1 on a level-count mismatch, 3 for a relaxation superoperator
 // that is not of Lindblad form (reg_cayley.hpp:146-155).
-MBG_HD int cay_precompute(const mat_in& m, int Nsolver, double* ws, double* out)
+template<class G>
+MBG_HD int cay_precompute(const mat_in& m, int Nsolver, double* ws, double* out, const G& g)
 {
     cay_layout L = make_cay_layout(Nsolver);
-    for (int i = 0; i < L.stride; i++) out[i] = 0.0;
-    write_fdtd(m, out);
+    for (int i = g.rank; i < L.stride; i += g.size) out[i] = 0.0;
+    g.sync();
+    if (g.rank == 0) write_fdtd(m, out);
     int N = Nsolver;
-    if (m.N == 0) {
-        out[L.has_qm] = 0.0;
-        return 0;
-    }
+    if (m.N == 0) return 0;
     if (m.N != Nsolver) return 1;
     if (m.relax_kind != 1) return 3;
-    out[L.has_qm] = 1.0;
-    const double kappa = m.dt / (2.0 * HBAR);
-    pack_hermitian(m.h_re, m.h_im, N, kappa, out + L.kH0);
-    pack_hermitian(m.mu_re, m.mu_im, N, kappa, out + L.kMu);
-    pack_hermitian(m.h_re, m.h_im, N, 1.0 / HBAR, out + L.W0);
-    pack_hermitian(m.mu_re, m.mu_im, N, m.carrier_density, out + L.Mn);
     double* X = ws;
     double* Fm = ws + N * N;
     double* W = ws + 2 * N * N;
-    for (int i = 0; i < N * N; i++) X[i] = m.S[i] * m.dt / 2;
-    expm_minus_identity(X, Fm, N, W);
-    for (int i = 0; i < N * N; i++) {
-        out[L.dD1 + i] = Fm[i];
-        out[L.d1 + i] = m.S[i];
+    for (int i = g.rank; i < N * N; i += g.size) X[i] = m.S[i] * m.dt / 2;
+    g.sync();
+    expm_minus_identity(X, Fm, N, W, g);
+    if (g.rank == 0) {
+        out[L.has_qm] = 1.0;
+        const double kappa = m.dt / (2.0 * HBAR);
+        pack_hermitian(m.h_re, m.h_im, N, kappa, out + L.kH0);
+        pack_hermitian(m.mu_re, m.mu_im, N, kappa, out + L.kMu);
+        pack_hermitian(m.h_re, m.h_im, N, 1.0 / HBAR, out + L.W0);
+        pack_hermitian(m.mu_re, m.mu_im, N, m.carrier_density, out + L.Mn);
+        for (int i = 0; i < N * N; i++) {
+            out[L.dD1 + i] = Fm[i];
+            out[L.d1 + i] = m.S[i];
+        }
+        for (int p = 0; p < L.P; p++) {
+            out[L.dD2 + p] = expm1(m.deph[p] * m.dt / 2);
+            out[L.d2 + p] = m.deph[p];
+        }
+        // initial density matrix (reg_cayley.hpp:269-272)
+        int rn = m.rho_levels;
+        for (int i = 0; i < N; i++) out[L.rho0 + i] = i < rn ? m.rho_diag[i] : 0.0;
+        for (int p = 0; p < L.P && p < m.rho_num_off; p++) {
+            out[L.rho0 + N + 2 * p] = m.rho_off_re[p];
+            out[L.rho0 + N + 2 * p + 1] = m.rho_off_im[p];
+        }
     }
-    for (int p = 0; p < L.P; p++) {
-        out[L.dD2 + p] = expm1(m.deph[p] * m.dt / 2);
-        out[L.d2 + p] = m.deph[p];
-    }
-    // initial density matrix (reg_cayley.hpp:269-272)
-    int rn = m.rho_levels;
-    for (int i = 0; i < N; i++) out[L.rho0 + i] = i < rn ? m.rho_diag[i] : 0.0;
-    for (int p = 0; p < L.P && p < m.rho_num_off; p++) {
-        out[L.rho0 + N + 2 * p] = m.rho_off_re[p];
-        out[L.rho0 + N + 2 * p + 1] = m.rho_off_im[p];
-    }
-    cay_polarisation_weights(L, out);
-    cay_free_step(L, ws, out);
+    g.sync();
+    cay_polarisation_weights(L, out, g);
+    cay_free_step(L, ws, out, g);
     return 0;
 }
 
