@@ -12,16 +12,19 @@
 // product is BF16 with K contiguous (16-byte aligned rows), each 16-byte
 // chunk is copied asynchronously (cp.async, zero-filled outside the
 // operand) into a ring of four stages filled two blocks ahead of the MMAs;
-// otherwise it is gathered with plain loads (any strides, FP32 or BF16,
-// converted to BF16 on the way) into two stages, each loaded while the
-// MMAs of the other run (the smaller footprint keeps four CTAs per SM for
-// the short-K gathers of training). One elected thread issues the MMAs;
+// otherwise a thread gathers a whole core matrix into registers (any
+// strides, FP32 or BF16, converted to BF16 on the way; 16-byte loads along
+// whichever dimension is contiguous, transposed in registers where that is
+// not K) while the MMAs of the block before run, and stores it into one of
+// two stages (the smaller footprint keeps four CTAs per SM for the short-K
+// products of training). One elected thread issues the MMAs;
 // tcgen05.commit arrives on the stage's mbarrier when they have read the
 // stage. Every wait is bounded: on time-out the kernel records it in the
 // status word and returns after freeing its TMEM.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <mutex>
@@ -44,20 +47,38 @@ constexpr int NTH = 128;         // 4 warps: warp w reads TMEM lanes 32w..32w+31
 constexpr int STAGES_ASYNC = 4, AHEAD_ASYNC = 2;
 constexpr int STAGES_SHORT = 2, AHEAD_SHORT = 2;
 constexpr int STAGES_GATHER = 2, AHEAD_GATHER = 0;
-constexpr int A_BYTES = BM * BK * 2;
-constexpr int B_BYTES = BN * BK * 2;
-constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-constexpr int smem_bytes(int stages) { return stages * STAGE_BYTES + 128; }  // + alignment slack
-static_assert(BM * (BN + 1) * 4 <= STAGES_GATHER * STAGE_BYTES, "epilogue tile must fit the stages");
 constexpr int TMEM_COLS = 64;    // power of two >= 32
-constexpr uint32_t LBO = 128;    // K-direction core-matrix stride (bytes)
-constexpr uint32_t SBO = 1024;   // M/N-direction 8-row-group stride (bytes)
+// Shared-memory strides of the core matrices (8 rows x 16 bytes) along K
+// (LBO) and along M/N (SBO). The asynchronous path packs them. On the
+// gather path a thread owns a whole core matrix and stores its rows one
+// after the other, so that a warp's store touches 32 core matrices: both
+// strides are a multiple of 128 bytes plus 16, which puts the 32 chunks in
+// different banks (packed, every lane's chunk would lie in the same four).
+template<bool GATHER>
+struct lay {
+    static constexpr uint32_t LBO = GATHER ? 144 : 128;
+    static constexpr uint32_t SBO = (BK / 8) * LBO + (GATHER ? 16 : 0);
+    static constexpr uint32_t A_BYTES = (BM / 8) * SBO;
+    static constexpr uint32_t B_BYTES = (BN / 8) * SBO;
+    static constexpr uint32_t STAGE_BYTES = A_BYTES + B_BYTES;
+    static constexpr int smem(int stages) { return (int) (stages * STAGE_BYTES) + 128; }  // + alignment slack
+};
+static_assert(BM * (BN + 1) * 4 <= STAGES_GATHER * lay<true>::STAGE_BYTES &&
+                  BM * (BN + 1) * 4 <= STAGES_SHORT * lay<false>::STAGE_BYTES,
+              "epilogue tile must fit the stages");
+// how the gather path reads an operand (chosen per segment by the host)
+enum : int32_t {
+    LD_ANY = 0,   // any strides: element by element
+    LD_K = 1,     // K contiguous, every row's 8-element chunks 16-byte aligned
+    LD_ROWS = 2   // rows contiguous, every 8 rows of a K entry 16-byte aligned
+};
 struct seg_t {
     const void* a;
     const void* b;
     int64_t a_sm, a_sk, a_sz;
     int64_t b_sn, b_sk, b_sz;
     int32_t k, a_type, b_type, neg;
+    int32_t a_ld, b_ld;  // LD_*
 };
 
 struct gemm_params {
@@ -66,6 +87,7 @@ struct gemm_params {
     seg_t seg[3];
     int32_t async_ok;  // every operand BF16, K contiguous, 16-byte aligned rows
     int32_t vec_c;     // STORE epilogue as 16-byte stores of 8 outputs along C's rows
+    int32_t vec4;      // the general epilogue by 4 consecutive outputs of a row
     int32_t vec_c2;    // the second output as 16-byte stores of 8 outputs along its columns
     int32_t fin;       // STORE mode without pre or gate: bias and activation applied once, on
                        // the way from TMEM into the shared tile
@@ -86,8 +108,6 @@ struct gemm_params {
 
 // ------------------------------------------------------------ helpers
 
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr) { return smem_desc_nsw(addr, LBO, SBO); }
-
 constexpr uint32_t IDESC = idesc_bf16(BM, BN);
 
 __device__ __forceinline__ float ld_elem(const void* base, int32_t type, int64_t off)
@@ -96,52 +116,117 @@ __device__ __forceinline__ float ld_elem(const void* base, int32_t type, int64_t
     return reinterpret_cast<const float*>(base)[off];
 }
 
-// Gather 8 consecutive K elements (k0 .. k0+7, global K index) of row `row`
-// of operand A (is_a) or B, negated for a negated segment's A, zero outside
-// the operand.
-__device__ __forceinline__ void gather_chunk(
-    const gemm_params& p, bool is_a, int z, int row, int rows, int k0, float (&v)[8])
+// One core matrix of an operand on the gather path: 8 rows (row0 ..) x 8
+// consecutive K entries (k0 ..), BF16, w[r] the 16 bytes of row r. All its
+// loads are 16 bytes wide where the operand is contiguous along K (LD_K: a
+// load is a row's chunk) or along its rows (LD_ROWS: a load is 8 rows of one
+// K entry, and the 8 x 8 block is transposed in registers); entries outside
+// the operand are zero. Element by element, the form before (96 loads a
+// thread and K block, each with its own type and bounds test), the products
+// of a training step (batch 64) took 23 to 122 us each, now 15 to 35 (caches
+// cold); the step 3.14 -> 1.40 ms.
+__device__ __forceinline__ void gather_unit(
+    const gemm_params& p, bool is_a, int z, int row0, int rows, int k0, uint32_t (&w)[8][4])
 {
 #pragma unroll
-    for (int e = 0; e < 8; e++) v[e] = 0.0f;
-    if (row < rows && k0 < p.ktotal) {
-        int s = 0;
-        if (p.nseg > 1 && k0 >= p.kstart[1]) s = 1;
-        if (p.nseg > 2 && k0 >= p.kstart[2]) s = 2;
-        const seg_t& g = p.seg[s];
-        const int kl = k0 - p.kstart[s];
-        const void* base = is_a ? g.a : g.b;
-        const int32_t type = is_a ? g.a_type : g.b_type;
-        const int64_t sr = is_a ? g.a_sm : g.b_sn;
-        const int64_t sk = is_a ? g.a_sk : g.b_sk;
-        const int64_t sz = is_a ? g.a_sz : g.b_sz;
-        const int64_t off = (int64_t) z * sz + (int64_t) row * sr + (int64_t) kl * sk;
-        const int nv = min(8, g.k - kl);
-        const size_t esz = type == MBG_BF16 ? 2 : 4;
-        const uintptr_t addr = reinterpret_cast<uintptr_t>(base) + (uintptr_t) (off * (int64_t) esz);
-        if (sk == 1 && nv == 8 && type == MBG_BF16 && (addr & 15) == 0) {
-            const uint4 q = *reinterpret_cast<const uint4*>(addr);
-            const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
+    for (int r = 0; r < 8; r++)
 #pragma unroll
-            for (int e = 0; e < 4; e++) {
-                const float2 f = __bfloat1622float2(h[e]);
-                v[2 * e] = f.x;
-                v[2 * e + 1] = f.y;
-            }
-        } else if (sk == 1 && nv == 8 && type == MBG_F32 && (addr & 15) == 0) {
-            const float4 a = reinterpret_cast<const float4*>(addr)[0];
-            const float4 b = reinterpret_cast<const float4*>(addr)[1];
-            v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-            v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+        for (int j = 0; j < 4; j++) w[r][j] = 0u;
+    if (row0 >= rows || k0 >= p.ktotal) return;
+    int s = 0;
+    if (p.nseg > 1 && k0 >= p.kstart[1]) s = 1;
+    if (p.nseg > 2 && k0 >= p.kstart[2]) s = 2;
+    const seg_t& g = p.seg[s];
+    const int kl = k0 - p.kstart[s];
+    const void* base = is_a ? g.a : g.b;
+    const int32_t type = is_a ? g.a_type : g.b_type;
+    const int32_t ld = is_a ? g.a_ld : g.b_ld;
+    const int64_t sr = is_a ? g.a_sm : g.b_sn;
+    const int64_t sk = is_a ? g.a_sk : g.b_sk;
+    const int64_t sz = is_a ? g.a_sz : g.b_sz;
+    const int64_t off = (int64_t) z * sz + (int64_t) row0 * sr + (int64_t) kl * sk;
+    const int nk = min(8, g.k - kl), nr = min(8, rows - row0);
+    if (ld == LD_K && nk == 8) {
+        if (type == MBG_BF16) {
+            const __nv_bfloat16* b = reinterpret_cast<const __nv_bfloat16*>(base) + off;
+#pragma unroll
+            for (int r = 0; r < 8; r++)
+                if (r < nr) {
+                    const uint4 q = __ldg(reinterpret_cast<const uint4*>(b + r * sr));
+                    w[r][0] = q.x;
+                    w[r][1] = q.y;
+                    w[r][2] = q.z;
+                    w[r][3] = q.w;
+                }
         } else {
+            const float* b = reinterpret_cast<const float*>(base) + off;
 #pragma unroll
-            for (int e = 0; e < 8; e++)
-                if (e < nv) v[e] = ld_elem(base, type, off + (int64_t) e * sk);
+            for (int r = 0; r < 8; r++)
+                if (r < nr) {
+                    const float4 x = __ldg(reinterpret_cast<const float4*>(b + r * sr));
+                    const float4 y = __ldg(reinterpret_cast<const float4*>(b + r * sr) + 1);
+                    w[r][0] = pack_bf16(x.x, x.y);
+                    w[r][1] = pack_bf16(x.z, x.w);
+                    w[r][2] = pack_bf16(y.x, y.y);
+                    w[r][3] = pack_bf16(y.z, y.w);
+                }
         }
-        if (g.neg && is_a) {  // negate the product: A only
+    } else if (ld == LD_ROWS && nr == 8) {
+        if (type == MBG_BF16) {
+            const __nv_bfloat16* b = reinterpret_cast<const __nv_bfloat16*>(base) + off;
+            uint32_t l[8][4];
 #pragma unroll
-            for (int e = 0; e < 8; e++) v[e] = -v[e];
+            for (int k = 0; k < 8; k++) {
+                uint4 q = make_uint4(0u, 0u, 0u, 0u);
+                if (k < nk) q = __ldg(reinterpret_cast<const uint4*>(b + k * sk));
+                l[k][0] = q.x;
+                l[k][1] = q.y;
+                l[k][2] = q.z;
+                l[k][3] = q.w;
+            }
+#pragma unroll
+            for (int r = 0; r < 8; r++)
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+                    w[r][j] = __byte_perm(l[2 * j][r >> 1], l[2 * j + 1][r >> 1], (r & 1) ? 0x7632 : 0x5410);
+        } else {
+            const float* b = reinterpret_cast<const float*>(base) + off;
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                float x[2][8];
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const int k = 2 * j + h;
+                    float4 u = make_float4(0.0f, 0.0f, 0.0f, 0.0f), v = u;
+                    if (k < nk) {
+                        u = __ldg(reinterpret_cast<const float4*>(b + k * sk));
+                        v = __ldg(reinterpret_cast<const float4*>(b + k * sk) + 1);
+                    }
+                    x[h][0] = u.x; x[h][1] = u.y; x[h][2] = u.z; x[h][3] = u.w;
+                    x[h][4] = v.x; x[h][5] = v.y; x[h][6] = v.z; x[h][7] = v.w;
+                }
+#pragma unroll
+                for (int r = 0; r < 8; r++) w[r][j] = pack_bf16(x[0][r], x[1][r]);
+            }
         }
+    } else {
+#pragma unroll
+        for (int r = 0; r < 8; r++) {
+            if (r >= nr) continue;
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const int64_t o = off + (int64_t) r * sr + (int64_t) (2 * j) * sk;
+                const float x = 2 * j < nk ? ld_elem(base, type, o) : 0.0f;
+                const float y = 2 * j + 1 < nk ? ld_elem(base, type, o + sk) : 0.0f;
+                w[r][j] = pack_bf16(x, y);
+            }
+        }
+    }
+    if (g.neg && is_a) {  // negate the product: A only
+#pragma unroll
+        for (int r = 0; r < 8; r++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) w[r][j] ^= 0x80008000u;
     }
 }
 
@@ -187,79 +272,83 @@ __device__ __forceinline__ void async_stage(
     }
 }
 
-// one 16-byte row of a core matrix, as BF16
-__device__ __forceinline__ void store_chunk(uint32_t dst, const float (&v)[8])
-{
-    const uint32_t w0 = pack_bf16(v[0], v[1]), w1 = pack_bf16(v[2], v[3]);
-    const uint32_t w2 = pack_bf16(v[4], v[5]), w3 = pack_bf16(v[6], v[7]);
-    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(w0), "r"(w1), "r"(w2), "r"(w3)
-                 : "memory");
-}
-
-// smem byte offset of the 16-byte chunk (row, kc) of a tile
-__device__ __forceinline__ uint32_t chunk_off(int row, int kc)
-{
-    return (uint32_t) (((row >> 3) * (BK / 8) + kc) * 128 + (row & 7) * 16);
-}
-
-constexpr int A_CHUNKS = BM * (BK / 8) / NTH;  // 8 per thread
-constexpr int B_CHUNKS = BN * (BK / 8) / NTH;  // 4 per thread
-
-// row and K chunk of chunk c: rows first when the operand's rows are
-// adjacent in memory (row stride 1), 16-byte K chunks first otherwise
-__device__ __forceinline__ void chunk_pos(int c, int R, bool rows_first, int& row, int& kc)
+// core matrix (8-row group rg, K group kg) of thread `t` of a tile of RG row
+// groups: K groups first where a load is a row's chunk (a warp reads 128
+// contiguous bytes of four row groups), row groups first where it is a run
+// of rows
+template<int RG>
+__device__ __forceinline__ void unit_pos(int t, bool rows_first, int& rg, int& kg)
 {
     if (rows_first) {
-        row = c % R;
-        kc = c / R;
+        rg = t % RG;
+        kg = t / RG;
     } else {
-        row = (c >> 6) * 8 + (c & 7);
-        kc = (c >> 3) & 7;
+        rg = t / (BK / 8);
+        kg = t % (BK / 8);
     }
 }
 
-// Stage the A (BM x BK) and B (BN x BK) tiles of K block kb: every global
-// load of the thread is issued before the first shared-memory store, so
-// that their latencies overlap.
-__device__ __forceinline__ void load_stage(
-    const gemm_params& p, int z, int m0, int n0, int kb, uint32_t sa, uint32_t sb)
+__device__ __forceinline__ void store_unit(uint32_t dst, const uint32_t (&w)[8][4])
+{
+#pragma unroll
+    for (int r = 0; r < 8; r++)
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst + 16u * r), "r"(w[r][0]), "r"(w[r][1]),
+                     "r"(w[r][2]), "r"(w[r][3])
+                     : "memory");
+}
+
+// the operands' core matrices of one K block held in registers between their
+// loads and the stage they go to: one of A per thread, one of B per thread of
+// the first two warps
+struct block_regs {
+    uint32_t a[8][4], b[8][4];
+};
+static_assert((BM / 8) * (BK / 8) == NTH && (BN / 8) * (BK / 8) == NTH / 2, "one core matrix per thread");
+
+__device__ __forceinline__ bool rows_first(const gemm_params& p, bool is_a, int kb)
 {
     const int k0 = kb * BK;
     int s = 0;
     if (p.nseg > 1 && k0 >= p.kstart[1]) s = 1;
     if (p.nseg > 2 && k0 >= p.kstart[2]) s = 2;
-    const bool a_rows = p.seg[s].a_sm == 1;
-    const bool b_rows = p.seg[s].b_sn == 1;
-    float va[A_CHUNKS][8], vb[B_CHUNKS][8];
-#pragma unroll
-    for (int i = 0; i < A_CHUNKS; i++) {
-        int row, kc;
-        chunk_pos(threadIdx.x + i * NTH, BM, a_rows, row, kc);
-        gather_chunk(p, true, z, m0 + row, p.m, k0 + kc * 8, va[i]);
+    return (is_a ? p.seg[s].a_sm : p.seg[s].b_sn) == 1;
+}
+
+__device__ __forceinline__ void load_block(const gemm_params& p, int z, int m0, int n0, int kb, block_regs& r)
+{
+    int rg, kg;
+    unit_pos<BM / 8>(threadIdx.x, rows_first(p, true, kb), rg, kg);
+    gather_unit(p, true, z, m0 + rg * 8, p.m, kb * BK + kg * 8, r.a);
+    if (threadIdx.x < NTH / 2) {
+        unit_pos<BN / 8>(threadIdx.x, rows_first(p, false, kb), rg, kg);
+        gather_unit(p, false, z, n0 + rg * 8, p.n, kb * BK + kg * 8, r.b);
     }
-#pragma unroll
-    for (int i = 0; i < B_CHUNKS; i++) {
-        int row, kc;
-        chunk_pos(threadIdx.x + i * NTH, BN, b_rows, row, kc);
-        gather_chunk(p, false, z, n0 + row, p.n, k0 + kc * 8, vb[i]);
+}
+
+__device__ __forceinline__ void store_block(const gemm_params& p, int kb, uint32_t sa, uint32_t sb, const block_regs& r)
+{
+    using L = lay<true>;
+    int rg, kg;
+    unit_pos<BM / 8>(threadIdx.x, rows_first(p, true, kb), rg, kg);
+    store_unit(sa + (uint32_t) rg * L::SBO + (uint32_t) kg * L::LBO, r.a);
+    if (threadIdx.x < NTH / 2) {
+        unit_pos<BN / 8>(threadIdx.x, rows_first(p, false, kb), rg, kg);
+        store_unit(sb + (uint32_t) rg * L::SBO + (uint32_t) kg * L::LBO, r.b);
     }
-#pragma unroll
-    for (int i = 0; i < A_CHUNKS; i++) {
-        int row, kc;
-        chunk_pos(threadIdx.x + i * NTH, BM, a_rows, row, kc);
-        store_chunk(sa + chunk_off(row, kc), va[i]);
-    }
-#pragma unroll
-    for (int i = 0; i < B_CHUNKS; i++) {
-        int row, kc;
-        chunk_pos(threadIdx.x + i * NTH, BN, b_rows, row, kc);
-        store_chunk(sb + chunk_off(row, kc), vb[i]);
-    }
+}
+
+// FP32 sums of 4 consecutive entries in one L2 operation
+__device__ __forceinline__ void red_add4(float* a, float4 v)
+{
+    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(a), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
+                 : "memory");
 }
 
 template<int STAGES, int AHEAD>
 __global__ void __launch_bounds__(NTH) gemm_kernel(const gemm_params p)
 {
+    constexpr bool GATHER = AHEAD == 0;  // only the asynchronous instantiations stage ahead
+    using L = lay<GATHER>;
     extern __shared__ __align__(128) uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t mbar[STAGES];
     __shared__ uint32_t tmem_sh;
@@ -294,14 +383,16 @@ __global__ void __launch_bounds__(NTH) gemm_kernel(const gemm_params p)
     fence_after();
     const uint32_t tmem = tmem_sh;
 
-    // stage block j: asynchronously where every operand allows it, else by
-    // plain loads (complete when the call returns)
+    // stage block j: by asynchronous copies, or (gather path) from the
+    // registers its loads went to while the MMAs of the block before ran
+    block_regs regs;
+    if constexpr (GATHER) load_block(p, z, m0, n0, kb0, regs);
     auto stage = [&](int j) {
-        const uint32_t sa = base + (uint32_t) ((j % STAGES) * STAGE_BYTES);
-        if (AHEAD > 0)  // only the asynchronous instantiation stages ahead
-            async_stage(p, z, m0, n0, kb0 + j, sa, sa + (uint32_t) A_BYTES);
+        const uint32_t sa = base + (uint32_t) (j % STAGES) * L::STAGE_BYTES;
+        if constexpr (!GATHER)
+            async_stage(p, z, m0, n0, kb0 + j, sa, sa + L::A_BYTES);
         else
-            load_stage(p, z, m0, n0, kb0 + j, sa, sa + (uint32_t) A_BYTES);
+            store_block(p, kb0 + j, sa, sa + L::A_BYTES, regs);
     };
     // exactly AHEAD copy groups before the loop (empty ones when there are
     // fewer blocks), so that waiting for all but the AHEAD most recent groups
@@ -328,16 +419,18 @@ __global__ void __launch_bounds__(NTH) gemm_kernel(const gemm_params p)
         if (fail_sh) break;
         if (tid == 0) {
             fence_after();
-            const uint32_t sa = base + (uint32_t) (st * STAGE_BYTES);
-            const uint32_t sb = sa + (uint32_t) A_BYTES;
+            const uint32_t sa = base + (uint32_t) st * L::STAGE_BYTES;
+            const uint32_t sb = sa + L::A_BYTES;
 #pragma unroll
             for (int kk = 0; kk < BK / 16; kk++) {
-                const uint64_t ad = smem_desc(sa + (uint32_t) (kk * 256));
-                const uint64_t bd = smem_desc(sb + (uint32_t) (kk * 256));
+                const uint64_t ad = smem_desc_nsw(sa + (uint32_t) kk * 2u * L::LBO, L::LBO, L::SBO);
+                const uint64_t bd = smem_desc_nsw(sb + (uint32_t) kk * 2u * L::LBO, L::LBO, L::SBO);
                 mma_bf16(tmem, ad, bd, IDESC, (it > 0 || kk > 0) ? 1u : 0u);
             }
             mma_commit(mb0 + 8u * st);
         }
+        if constexpr (GATHER)
+            if (it + 1 < nit) load_block(p, z, m0, n0, kb0 + it + 1, regs);
     }
     cp_async_wait<0>();  // no copy outlives the loop (a break leaves some in flight)
 
@@ -428,8 +521,50 @@ __global__ void __launch_bounds__(NTH) gemm_kernel(const gemm_params p)
                 }
             }
         }
+        if (p.vec4) {
+            // the general epilogue (bias, pre, gate, accumulate, atomic) on 4
+            // consecutive outputs of a row: 16-byte accesses of C, pre and
+            // gate (8-byte of a BF16 C), one L2 operation per 4 sums
 #pragma unroll 1
-        for (int e = (p.vec_c || p.rowdot) ? BM * BN : tid; e < BM * BN; e += NTH) {
+            for (int e = tid; e < BM * (BN / 4); e += NTH) {
+                const int r = e / (BN / 4), c0 = (e % (BN / 4)) * 4;
+                const int row = m0 + r, col = n0 + c0;
+                if (row >= p.m || col >= p.n) continue;  // n is a multiple of 4
+                const int64_t off = (int64_t) z * p.c_sz + (int64_t) row * p.c_sm + col;
+                float v[4];
+#pragma unroll
+                for (int i = 0; i < 4; i++) v[i] = p.alpha * tile[r * LD + c0 + i];
+                if (p.mode == MBG_GEMM_ATOMIC) {
+                    red_add4(reinterpret_cast<float*>(p.c) + off, make_float4(v[0], v[1], v[2], v[3]));
+                    continue;
+                }
+                if (p.mode == MBG_GEMM_ACCUM)
+#pragma unroll
+                    for (int i = 0; i < 4; i++) v[i] += ld_elem(p.c, p.c_type, off + i);
+                if (p.bias)
+#pragma unroll
+                    for (int i = 0; i < 4; i++) v[i] += p.bias[col + i];
+                if (p.pre) *reinterpret_cast<float4*>(p.pre + off) = make_float4(v[0], v[1], v[2], v[3]);
+                if (p.act == MBG_ACT_GELU) {
+#pragma unroll
+                    for (int i = 0; i < 4; i++) v[i] = gelu(v[i]);
+                } else if (p.act == MBG_ACT_GELU_BWD) {
+                    const float4 gt = *reinterpret_cast<const float4*>(p.gate + off);
+                    v[0] *= gelu_grad(gt.x);
+                    v[1] *= gelu_grad(gt.y);
+                    v[2] *= gelu_grad(gt.z);
+                    v[3] *= gelu_grad(gt.w);
+                }
+                if (p.c_type == MBG_BF16)
+                    *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p.c) + off) =
+                        make_uint2(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]));
+                else
+                    *reinterpret_cast<float4*>(reinterpret_cast<float*>(p.c) + off) =
+                        make_float4(v[0], v[1], v[2], v[3]);
+            }
+        }
+#pragma unroll 1
+        for (int e = (p.vec_c || p.vec4 || p.rowdot) ? BM * BN : tid; e < BM * BN; e += NTH) {
             const int r = rows_fast ? e % BM : e / BN;
             const int cc = rows_fast ? e / BM : e % BN;
             const int row = m0 + r, col = n0 + cc;
@@ -553,20 +688,35 @@ __global__ void image_kernel(const float* x, int batch, int rows, int cols, int6
     }
 }
 
-// one CTA per (column, row slice): strided partial sums, then atomics
-__global__ void colsum_kernel(const float* x, int64_t rows, int cols, int64_t rs, float* out)
+// Column sums: a CTA takes 32 columns and a slice of the rows, a warp one
+// row at a time (32 adjacent columns: one coalesced read), the warps' partial
+// sums meet in shared memory, one atomic per column. (One column per CTA read
+// a 32-byte sector for every 4 bytes and every column again: 19.7 us for
+// 65,536 x 64, now 8.2 us, caches cold.)
+__global__ void __launch_bounds__(256) colsum_kernel(const float* x, int64_t rows, int cols, int64_t rs, float* out)
 {
-    const int col = blockIdx.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int col = blockIdx.x * 32 + lane;
     float s = 0.0f;
-    for (int64_t r = blockIdx.y * (int64_t) blockDim.x + threadIdx.x; r < rows; r += (int64_t) gridDim.y * blockDim.x)
-        s += x[r * rs + col];
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    __shared__ float part[32];
-    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
+    if (col < cols) {
+        const int64_t step = (int64_t) gridDim.y * nw;
+        int64_t r = (int64_t) blockIdx.y * nw + warp;
+        float s1 = 0.0f, s2 = 0.0f, s3 = 0.0f;
+        for (; r + 3 * step < rows; r += 4 * step) {
+            s += x[r * rs + col];
+            s1 += x[(r + step) * rs + col];
+            s2 += x[(r + 2 * step) * rs + col];
+            s3 += x[(r + 3 * step) * rs + col];
+        }
+        for (; r < rows; r += step) s += x[r * rs + col];
+        s = (s + s1) + (s2 + s3);
+    }
+    __shared__ float part[8][32];
+    part[warp][lane] = s;
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (warp == 0 && col < cols) {
         float t = 0.0f;
-        for (int w = 0; w < (int) (blockDim.x >> 5); w++) t += part[w];
+        for (int w = 0; w < nw; w++) t += part[w][lane];
         atomicAdd(out + col, t);
     }
 }
@@ -668,6 +818,19 @@ void require(bool c, const char* msg)
     if (!c) throw std::invalid_argument(msg);
 }
 
+// Whether the gather path can read an operand by 16-byte loads along K or
+// along its rows: that dimension contiguous, every other stride and the
+// base multiples of 16 bytes (a core matrix starts at a multiple of 8 rows
+// and, within its segment, of 8 K entries).
+int32_t load_form(const void* base, int32_t type, int64_t sr, int64_t sk, int64_t sz)
+{
+    const int64_t w = type == MBG_BF16 ? 8 : 4;
+    if ((reinterpret_cast<uintptr_t>(base) & 15) != 0 || sz % w != 0) return LD_ANY;
+    if (sk == 1 && sr % w == 0) return LD_K;
+    if (sr == 1 && sk % w == 0) return LD_ROWS;
+    return LD_ANY;
+}
+
 void gemm(const mbg_gemm_desc* d, cudaStream_t s)
 {
     require(d != nullptr, "gemm: null descriptor");
@@ -697,7 +860,8 @@ void gemm(const mbg_gemm_desc* d, cudaStream_t s)
         p.kstart[i] = kt;
         kt += g.k;
         p.seg[i] = seg_t{ g.a, g.b, g.a_sm, g.a_sk, g.a_sz, g.b_sn, g.b_sk, g.b_sz, g.k, g.a_type, g.b_type,
-                          g.negate };
+                          g.negate, load_form(g.a, g.a_type, g.a_sm, g.a_sk, g.a_sz),
+                          load_form(g.b, g.b_type, g.b_sn, g.b_sk, g.b_sz) };
     }
     p.kstart[d->nseg] = kt;
     p.ktotal = kt;
@@ -733,6 +897,12 @@ void gemm(const mbg_gemm_desc* d, cudaStream_t s)
     p.rowdot = d->rowdot;
     p.rowdot_bias = d->rowdot_bias;
     if (p.rowdot) p.vec_c = 0;
+    // the general epilogue by fours: rows contiguous in C (and so in pre and
+    // gate, which share its strides), every group of 4 aligned and whole
+    const uintptr_t c4 = d->c_type == MBG_BF16 ? 7 : 15;
+    p.vec4 = !p.vec_c && !p.rowdot && d->c_sn == 1 && d->c_sm % 4 == 0 && d->c_sz % 4 == 0 && d->n % 4 == 0 &&
+        !plain_store && (reinterpret_cast<uintptr_t>(d->c) & c4) == 0 &&
+        (reinterpret_cast<uintptr_t>(d->pre) & 15) == 0 && (reinterpret_cast<uintptr_t>(d->gate) & 15) == 0;
     p.fin = plain_store ? 1 : 0;
     p.c = d->c;
     p.c_sm = d->c_sm;
@@ -756,21 +926,21 @@ void gemm(const mbg_gemm_desc* d, cudaStream_t s)
     static std::once_flag attr;
     std::call_once(attr, [] {
         cudaFuncSetAttribute(gemm_kernel<STAGES_ASYNC, AHEAD_ASYNC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             smem_bytes(STAGES_ASYNC));
+                             lay<false>::smem(STAGES_ASYNC));
         cudaFuncSetAttribute(gemm_kernel<STAGES_GATHER, AHEAD_GATHER>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             smem_bytes(STAGES_GATHER));
+                             lay<true>::smem(STAGES_GATHER));
         cudaFuncSetAttribute(gemm_kernel<STAGES_SHORT, AHEAD_SHORT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             smem_bytes(STAGES_SHORT));
+                             lay<false>::smem(STAGES_SHORT));
     });
     const dim3 grid((unsigned) tiles, (unsigned) ysplits, (unsigned) d->batch);
     // (with at most AHEAD_SHORT = STAGES_SHORT blocks every block is staged
     // before the loop, so no stage is ever reused)
     if (p.async_ok && p.kblocks_per_split <= STAGES_SHORT)
-        gemm_kernel<STAGES_SHORT, AHEAD_SHORT><<<grid, NTH, smem_bytes(STAGES_SHORT), s>>>(p);
+        gemm_kernel<STAGES_SHORT, AHEAD_SHORT><<<grid, NTH, lay<false>::smem(STAGES_SHORT), s>>>(p);
     else if (p.async_ok)
-        gemm_kernel<STAGES_ASYNC, AHEAD_ASYNC><<<grid, NTH, smem_bytes(STAGES_ASYNC), s>>>(p);
+        gemm_kernel<STAGES_ASYNC, AHEAD_ASYNC><<<grid, NTH, lay<false>::smem(STAGES_ASYNC), s>>>(p);
     else
-        gemm_kernel<STAGES_GATHER, AHEAD_GATHER><<<grid, NTH, smem_bytes(STAGES_GATHER), s>>>(p);
+        gemm_kernel<STAGES_GATHER, AHEAD_GATHER><<<grid, NTH, lay<true>::smem(STAGES_GATHER), s>>>(p);
     check_launch("gemm_kernel");
 }
 
@@ -824,10 +994,10 @@ int mbg_fno_colsum(const float* x, int64_t rows, int32_t cols, int64_t row_strid
 {
     return guard([&] {
         require(x && out && rows > 0 && cols > 0 && cols <= 65535 && row_stride >= cols, "colsum: bad arguments");
-        int ys = (int) ((rows + 255) / 256);
-        if (ys > 64) ys = 64;
-        colsum_kernel<<<dim3((unsigned) cols, (unsigned) ys), 256, 0, (cudaStream_t) stream>>>(x, rows, cols,
-                                                                                            row_stride, out);
+        // 64 rows a CTA at least, two CTAs per SM at most
+        const unsigned xs = (unsigned) ((cols + 31) / 32);
+        const int64_t ys = std::max<int64_t>(1, std::min<int64_t>((rows + 63) / 64, 304 / xs));
+        colsum_kernel<<<dim3(xs, (unsigned) ys), 256, 0, (cudaStream_t) stream>>>(x, rows, cols, row_stride, out);
         check_launch("colsum_kernel");
     });
 }

@@ -16,7 +16,7 @@ with fixed BF16 bases. Master weights, gradients and Adam moments are FP32
 in one flat buffer each. torch provides device memory and the stream only.
 
 Layouts (row-major, element strides): activations v_l [B, S, W] BF16,
-pre-activations [B, S, W] FP32, spectra Vh [B, W, 2 Mo] FP32 (Re modes then
+pre-activations [B, S, W] FP32, spectra Vh [B, 2 Mo, W] FP32 (Re modes then
 Im modes), mixed spectra Y [B, Mo, 2 W] FP32, mode blocks [Mo, 2W, 2W] BF16.
 """
 import math
@@ -199,16 +199,16 @@ class FNO:
                b["v"][0], 0, W, 1, bias=p["bp"])
         for l in range(L):
             v, vh = b["v"][l], b["Vh"][l]
-            # truncated DFT: Vh[b, c, m'] = sum_s F[m', s] v[b, s, c]
+            # truncated DFT: Vh[b, m', c] = sum_s F[m', s] v[b, s, c]
             vh.zero_()
-            K.gemm(W, 2 * Mo, [Seg(v, 0, 1, W, S * W, self.F, 0, S, 1, 0, S)],
-                   vh, 0, 2 * Mo, 1, W * 2 * Mo, batch=B,
+            K.gemm(2 * Mo, W, [Seg(self.F, 0, S, 1, 0, v, 0, 1, W, S * W, S)],
+                   vh, 0, W, 1, 2 * Mo * W, batch=B,
                    mode=T.MBG_GEMM_ATOMIC, split_k=self.DFT_SPLIT)
             # mode mixing, per mode m: Y[b, m, :] = blk[m] [Re; Im]
             blk = self.blk[l]
             K.gemm(B, 2 * W,
-                   [Seg(vh, 0, W * 2 * Mo, 2 * Mo, 1, blk, 0, 2 * W, 1, 4 * W * W, W),
-                    Seg(vh, Mo, W * 2 * Mo, 2 * Mo, 1, blk, W, 2 * W, 1, 4 * W * W, W)],
+                   [Seg(vh, 0, 2 * Mo * W, 1, W, blk, 0, 2 * W, 1, 4 * W * W, W),
+                    Seg(vh, Mo * W, 2 * Mo * W, 1, W, blk, W, 2 * W, 1, 4 * W * W, W)],
                    b["Y"], 0, Mo * 2 * W, 1, 2 * W, batch=Mo)
             # inverse DFT + pointwise path + bias (+ GELU), per sample
             last = l == L - 1
@@ -458,16 +458,16 @@ class FNO:
                    mode=T.MBG_GEMM_ATOMIC, split_k=self.DFT_SPLIT)
             dY = b["dY"]
             a_re = dict(a_sm=1, a_sk=2 * Mo * W, a_sz=W)
-            b_v = dict(b_sn=2 * Mo, b_sk=W * 2 * Mo, b_sz=1)
+            b_v = dict(b_sn=1, b_sk=2 * Mo * W, b_sz=W)
 
             def sg(a_off, b_off, neg=False):
                 return Seg(dY, a_off, a_re["a_sm"], a_re["a_sk"], a_re["a_sz"],
                            vh, b_off, b_v["b_sn"], b_v["b_sk"], b_v["b_sz"], B,
                            negate=neg)
             # spectral weights, per mode
-            K.gemm(W, W, [sg(0, 0), sg(Mo * W, Mo)],
+            K.gemm(W, W, [sg(0, 0), sg(Mo * W, Mo * W)],
                    g["wr%d" % l], 0, 1, W, W * W, batch=Mo)
-            K.gemm(W, W, [sg(0, Mo, True), sg(Mo * W, 0)],
+            K.gemm(W, W, [sg(0, Mo * W, True), sg(Mo * W, 0)],
                    g["wi%d" % l], 0, 1, W, W * W, batch=Mo)
             # spectra: dVh = blk^T dY, Re and Im halves, per mode
             for half in range(2):
@@ -475,11 +475,11 @@ class FNO:
                        [Seg(dY, 0, 2 * Mo * W, 1, W, blk, half * W, 1, 2 * W, 4 * W * W, W),
                         Seg(dY, Mo * W, 2 * Mo * W, 1, W, blk, 2 * W * W + half * W, 1, 2 * W,
                             4 * W * W, W)],
-                       b["dVh"], half * Mo, W * 2 * Mo, 2 * Mo, 1, batch=Mo)
+                       b["dVh"], half * Mo * W, 2 * Mo * W, 1, W, batch=Mo)
             # activations: dv = F^T dVh + dpre W_l, then GELU'
             nxt = 1 - cur
             K.gemm(S, W,
-                   [Seg(self.F, 0, 1, S, 0, b["dVh"], 0, 2 * Mo, 1, W * 2 * Mo, 2 * Mo),
+                   [Seg(self.F, 0, 1, S, 0, b["dVh"], 0, 1, W, 2 * Mo * W, 2 * Mo),
                     Seg(dpre, 0, W, 1, S * W, p["W%d" % l], 0, 1, W, 0, W)],
                    b["dpre"][nxt], 0, W, 1, S * W, batch=B,
                    act=T.MBG_ACT_GELU_BWD if l > 0 else T.MBG_ACT_NONE,
