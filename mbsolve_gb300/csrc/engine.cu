@@ -1535,7 +1535,9 @@ private:
     // the unfilled part of their last wave of tiles; the persistent kernel
     // does not. Where the persistent kernel will run, rank the depths by
     // their rate divided by that wave efficiency, tiles / (ceil(tiles /
-    // slots) * slots): one 65,536-point 6-level run measured 8.4e9
+    // slots) * slots), where there is more than one wave (fewer tiles than
+    // slots leave slots idle in either kernel: a level waits for the one
+    // before): one 65,536-point 6-level run measured 8.4e9
     // cell-updates/s persistent at depth 8 (launch per level 5.8e9, 1.29
     // waves) and 8.0e9 at depth 16 (6.3e9, 1.50 waves), which this ranks
     // 9.0 vs 8.4.
@@ -1555,7 +1557,7 @@ private:
             const double n = (double) ntiles[i];
             if (depths[i].second <= 0 || n <= 0) continue;
             if (forced < 0 && n >= 4 * slots) continue;  // would not run persistent
-            const double eff = n / (std::ceil(n / slots) * slots);
+            const double eff = n <= slots ? 1.0 : n / (std::ceil(n / slots) * slots);
             const double est = depths[i].second / eff;
             if (est > top) {
                 top = est;
@@ -1595,21 +1597,36 @@ private:
                 }
             }
             if (!cached) {
-                // stage 1: launch shape at the default depth; stage 2: depth
-                // (each stage ends with a run-off of its close contenders)
+                // stage 1: launch shape, at the default depth or (few grid
+                // points: launches of tens of microseconds) at every depth,
+                // because shapes that leave most of the chip idle differ in
+                // the depth they need (16,384 2-level points, FP32: 2 x 128
+                // is best at depth 64 with 0.52 us a step, third at 16 with
+                // 0.98, where 1 x 128 leads with 0.87); stage 2: depth of the
+                // best shape (each stage ends with a run-off of its close
+                // contenders)
+                const int depth_list[] = { 1, 2, 4, 8, 16, 32, 64 };
+                const bool joint = cells_ <= (1u << 17);
                 std::vector<std::pair<tuning, double> > shapes;
                 for (const auto& e : kernel_registry<T>()) {
                     if (e.algo != kind_.algo || e.lev != kind_.N || e.staging != staging_ || !e.fn) continue;
-                    tuning c = t;
-                    c.C = e.C;
-                    c.NT = e.NT;
-                    if (align_halo(c.depth) * 4 > c.C * c.NT) continue;
-                    shapes.push_back({ c, time_candidate(c) });
+                    for (int d : depth_list) {
+                        tuning c = t;
+                        c.C = e.C;
+                        c.NT = e.NT;
+                        if (joint)
+                            c.depth = d;
+                        else if (d != depth_list[0])
+                            continue;  // the default depth, once
+                        if (align_halo(c.depth) * 4 > c.C * c.NT) continue;
+                        if (joint && d > 1 && (uint64_t) d > nt_max_) continue;
+                        shapes.push_back({ c, time_candidate(c) });
+                    }
                 }
                 tuning best = shapes.empty() ? t : runoff(shapes, 0.10);
                 std::vector<std::pair<tuning, double> > depths;
                 std::vector<size_t> ntiles;
-                for (int d : { 1, 2, 4, 8, 16, 32, 64 }) {
+                for (int d : depth_list) {
                     tuning c = best;
                     c.depth = d;
                     if (align_halo(d) * 4 > c.C * c.NT) continue;

@@ -639,11 +639,9 @@ __device__ __forceinline__ void df_h_update(float& hh, float& hl, float dh, floa
     hl = e2 - (hh - s);
 }
 
-// hi + lo += v (v in FP64)
-__device__ __forceinline__ void df_add(float& hh, float& hl, double v)
+// hi + lo += vh + vl
+__device__ __forceinline__ void df_add(float& hh, float& hl, float vh, float vl)
 {
-    const float vh = (float) v;
-    const float vl = (float) (v - (double) vh);
     const float s = hh + vh;
     const float bv = s - hh;
     const float err = (hh - (s - bv)) + (vh - bv);

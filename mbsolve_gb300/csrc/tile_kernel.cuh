@@ -11,7 +11,6 @@
 #include "kernels.cuh"
 #include "tc_density.cuh"
 #include "bulk_stage.cuh"
-#include "pair_steps.cuh"
 
 namespace mbg {
 
@@ -24,41 +23,228 @@ struct density_len {
 constexpr int TILE_MAX_SRC = 8;
 constexpr int TILE_MAX_REC = 8;
 constexpr int TILE_MAX_STEPS = 256;  // the largest temporal depth
+constexpr int TILE_SRC_VALUES = 256; // source values staged per launch
 
 struct no_coef {
     __device__ __forceinline__ explicit no_coef(const void*) {}
 };
 
+// What the tile's threads need of its sources and records in the time loop,
+// prepared once per launch. The loop itself then spends two instructions a
+// step on them in the threads that own no source point and no due record:
+// the tiles of a single run wait for the slowest, and a step of the tile
+// that recorded a probe took three times a plain one's time (2-level FP32
+// run of 16,384 points with two probes, a source and two full-grid records,
+// 2 points x 128 threads, depth 64: 1.08 us a step, 0.34 without them; now
+// 0.52).
 struct tile_lists {
     int nsrc, nrec, overflow;
-    int wall;  // the window holds a mirror wall (run_desc k_left, k_right)
+    int wall;    // the window holds a mirror wall (run_desc k_left, k_right)
+    int staged;  // src_values holds the sources' values (step m of source s at s * nsteps + m)
     src_desc src[TILE_MAX_SRC];
     rec_desc rec[TILE_MAX_REC];
-    // steps of the launch at which each record takes a row, one bit a step
-    uint32_t due[TILE_MAX_REC][TILE_MAX_STEPS / 32];
-    __device__ __forceinline__ bool is_due(int r, int m) const { return (due[r][m >> 5] >> (m & 31)) & 1u; }
+    uint8_t due[TILE_MAX_STEPS];  // per step: the records that take a row, one bit each
+    // the same per record, one bit a step, to count rows from
+    uint32_t mask[TILE_MAX_REC][TILE_MAX_STEPS / 32];
+    uint64_t row0[TILE_MAX_REC];  // floor(ratio * first step)
+    // row of the due step m, floor(ratio * step): the floor goes up by one
+    // at every due step after the launch's first
+    __device__ __forceinline__ uint64_t row(int r, int m) const
+    {
+        uint32_t c = __popc(mask[r][m >> 5] << (31 - (m & 31)));
+        for (int w = 0; w < (m >> 5); w++) c += __popc(mask[r][w]);
+        return row0[r] + c - (mask[r][0] & 1u);
+    }
 };
 
-// Fills tl.due, the reference's predicate (hasto_record) once per launch
-// and step instead of once per step in every thread: it takes about ten
-// FP64 instructions a record, each 64 cycles of a scheduler's FP64 unit, in
-// FP32 kernels too. Runs with two full-grid records: 2-level FP32, 16,384
-// points, 3.57 -> 2.41 ms per 2,000 steps; 6-level FP32, 65,536 points,
-// 5.23 -> 4.39 ms per 500; 3-level Lambda, 1,048,576 points, 16.8 -> 13.6
-// ms per 200. Every thread calls it; a barrier follows.
-template<int NT>
-__device__ __forceinline__ void mark_due(tile_lists& tl, uint64_t step0, int nsteps)
+// the sources' values, as the kernels apply them: the value, and the rest
+// of the FP64 value where the fields are float pairs
+template<typename T>
+struct src_values {
+    T hi[TILE_SRC_VALUES];
+    T lo[sizeof(T) == 4 ? TILE_SRC_VALUES : 1];
+};
+
+// Fills the schedules and the sources' values; every thread calls it, a
+// barrier follows. The reference's predicate (hasto_record) runs once per
+// launch and step instead of once per step in every thread: about ten FP64
+// instructions a record, each 64 cycles of a scheduler's FP64 unit (runs
+// with two full-grid records: 2-level FP32, 16,384 points, 3.57 -> 2.41 ms
+// per 2,000 steps; 6-level FP32, 65,536 points, 5.23 -> 4.39 ms per 500;
+// 3-level Lambda, 1,048,576 points, 16.8 -> 13.6 ms per 200).
+template<typename T, int NT>
+__device__ __forceinline__ void prepare_lists(const kparams<T>& p, tile_lists& tl, src_values<T>& sv, uint64_t step0,
+                                              int nsteps)
 {
-    for (int r = 0; r < tl.nrec; r++) {
-        const double ratio = tl.rec[r].ratio;
+    if (tl.overflow) return;
+    if (p.record) {
         for (int w = threadIdx.x >> 5; w * 32 < nsteps; w += NT / 32) {
-            const int m = w * 32 + (int) (threadIdx.x & 31);
-            const bool b = m < nsteps && (ratio == 1.0 || hasto_record(ratio, step0 + (uint64_t) m));
-            const uint32_t mask = __ballot_sync(0xffffffffu, b);
-            if ((threadIdx.x & 31) == 0) tl.due[r][w] = mask;
+            const int lane = threadIdx.x & 31, m = w * 32 + lane;
+            uint32_t mine = 0;
+            for (int r = 0; r < tl.nrec; r++) {
+                const double ratio = tl.rec[r].ratio;
+                const bool b = m < nsteps && (ratio == 1.0 || hasto_record(ratio, step0 + (uint64_t) m));
+                const uint32_t word = __ballot_sync(0xffffffffu, b);
+                if (lane == 0) tl.mask[r][w] = word;
+                mine |= b ? 1u << r : 0u;
+            }
+            tl.due[m] = (uint8_t) mine;
+        }
+        if (threadIdx.x < tl.nrec) {
+            const double ratio = tl.rec[threadIdx.x].ratio;
+            tl.row0[threadIdx.x] = ratio == 1.0 ? step0 : (uint64_t) floor(ratio * (double) step0);
         }
     }
+    if (tl.staged)
+        for (int i = threadIdx.x; i < tl.nsrc * nsteps; i += NT) {
+            const int k = i / nsteps;
+            const double v = p.stab[tl.src[k].table_offset + step0 + (uint64_t) (i - k * nsteps)];
+            sv.hi[i] = (T) v;
+            if constexpr (sizeof(T) == 4) sv.lo[i] = (T) (v - (double) (T) v);
+        }
 }
+
+// The sources and records of one thread's points. Held in registers: a load
+// of the lists at the end of every step, where nothing is left to hide it,
+// costs a lone warp 0.1 us of its 0.4 us step. A thread's only source, and
+// the first single-point field record among its points, are prepared to
+// their last index, so that a step applies them with a handful of
+// instructions (through the lists 430 and 700 cycles of the owner's warp).
+constexpr uint32_t OWN_ALL = 0xffffffffu;
+
+template<typename T>
+struct tile_own {
+    uint32_t bits;  // sources (bits 0 ..), records (bits 8 ..); OWN_ALL: more than a tile lists
+    int32_t src;    // -1, or the only source: first value | point << 16 | type << 24
+    int32_t rec;    // -1, or the field record: index | point << 8 | type << 16
+    uint32_t left;  // its rows from here on
+    T* dst;         // its next row
+};
+
+// after prepare_lists and a barrier
+template<typename T, int C>
+__device__ __forceinline__ tile_own<T> own_lists(const kparams<T>& p, const tile_lists& tl, const tile_desc& td,
+                                                 int64_t l0, int nsteps)
+{
+    tile_own<T> own{ 0u, -1, -1, 0u, nullptr };
+    if (tl.overflow) {
+        own.bits = OWN_ALL;
+        return own;
+    }
+    int count = 0;
+    for (int k = 0; k < tl.nsrc; k++) {
+        const int64_t jj = (int64_t) tl.src[k].x_idx - l0;
+        if (jj < 0 || jj >= C) continue;
+        own.bits |= 1u << k;
+        own.src = k * nsteps | (int) jj << 16 | tl.src[k].type << 24;
+        count++;
+    }
+    if (count != 1 || !tl.staged) own.src = -1;
+    for (int r = 0; p.record && r < tl.nrec; r++) {
+        const rec_desc& rc = tl.rec[r];
+        const int64_t lo = max((int64_t) rc.pos, (int64_t) td.out_start);
+        const int64_t hi = min((int64_t) rc.pos + rc.cols, (int64_t) td.out_start + td.out_len);
+        if (l0 + C <= lo || l0 >= hi) continue;
+        own.bits |= 256u << r;
+        if (own.rec < 0 && rc.cols == 1 && rc.type <= 2) {
+            // the row of the launch's first due step
+            const uint64_t row = tl.row0[r] + (tl.mask[r][0] & 1u ? 0u : 1u);
+            own.rec = r | (int) (lo - l0) << 8 | rc.type << 16;
+            own.dst = p.scratch + rc.offset + row;
+            own.left = row < rc.rows ? (uint32_t) min(rc.rows - row, (uint64_t) 0xffffffffu) : 0u;
+        }
+    }
+    return own;
+}
+
+// f(point, type, value, rest of the value) for each source of `own` at step
+// m (absolute step n)
+template<typename T, class F>
+__device__ __forceinline__ void for_sources(const kparams<T>& p, const run_desc& rd, const tile_lists& tl,
+                                            const src_values<T>& sv, const tile_own<T>& own, int64_t l0, int m,
+                                            int nsteps, uint64_t n, F&& f)
+{
+    if ((own.bits & 255u) == 0u) return;
+    if (own.src >= 0) {
+        const int i = (own.src & 0xffff) + m;
+        f((own.src >> 16) & 255, own.src >> 24, sv.hi[i], sizeof(T) == 4 ? sv.lo[sizeof(T) == 4 ? i : 0] : T(0));
+        return;
+    }
+    uint32_t todo = own.bits & 255u;
+    const bool all = own.bits == OWN_ALL;
+    const int end = (int) (rd.src_end - rd.src_begin);
+    for (int k = 0; all ? k < end : todo != 0u; k++) {
+        if (!all) {
+            k = __ffs(todo) - 1;
+            todo &= todo - 1u;
+        }
+        const src_desc sd = all ? p.srcs[rd.src_begin + k] : tl.src[k];
+        T h, l = T(0);
+        if (tl.staged) {
+            h = sv.hi[k * nsteps + m];
+            if constexpr (sizeof(T) == 4) l = sv.lo[k * nsteps + m];
+        } else {
+            const double v = p.stab[sd.table_offset + n];
+            h = (T) v;
+            if constexpr (sizeof(T) == 4) l = (T) (v - (double) h);
+        }
+        const int64_t jj = (int64_t) sd.x_idx - l0;
+        f(jj >= 0 && jj < 255 ? (int) jj : 255, sd.type, h, l);  // 255: no point of any thread
+    }
+}
+
+// the records of `own` that take a row at step m (asked at the start of a
+// step, used at its end)
+template<typename T>
+__device__ __forceinline__ uint32_t due_records(const kparams<T>& p, const tile_lists& tl, const tile_own<T>& own, int m)
+{
+    return own.bits == OWN_ALL ? (uint32_t) p.record : own.bits > 255u ? (own.bits >> 8) & tl.due[m] : 0u;
+}
+
+// Takes the rows of the records `todo` (due_records) at step m (absolute step
+// n): field(point, type) is a field value (types 0 to 2), f(record, row) any
+// other record's row.
+template<typename T, class V, class F>
+__device__ __forceinline__ void for_records(const kparams<T>& p, const run_desc& rd, const tile_lists& tl,
+                                            tile_own<T>& own, uint32_t todo, int m, uint64_t n, V&& field, F&& f)
+{
+    if (todo == 0u) return;
+    const bool all = own.bits == OWN_ALL;
+    if (own.rec >= 0) {
+        const uint32_t bit = 1u << (own.rec & 255);
+        if (todo & bit) {
+            todo &= ~bit;
+            const T v = field((own.rec >> 8) & 255, own.rec >> 16);
+            if (own.left) *own.dst = v;
+            own.left -= own.left ? 1u : 0u;
+            own.dst++;
+            if (!isfinite(v)) atomicOr(p.status, STATUS_NONFINITE);
+        }
+        if (todo == 0u) return;
+    }
+    const int end = (int) (rd.rec_end - rd.rec_begin);
+    for (int r = 0; all ? r < end : todo != 0u; r++) {
+        if (!all) {
+            r = __ffs(todo) - 1;
+            todo &= todo - 1u;
+        }
+        const rec_desc rc = all ? p.recs[rd.rec_begin + r] : tl.rec[r];
+        uint64_t row;
+        if (all) {
+            if (rc.ratio != 1.0 && !hasto_record(rc.ratio, n)) continue;
+            row = rc.ratio == 1.0 ? n : (uint64_t) floor(rc.ratio * (double) n);
+        } else {
+            row = tl.row(r, m);
+        }
+        if (row < rc.rows) f(rc, row);
+    }
+}
+
+}  // namespace mbg
+
+#include "pair_steps.cuh"
+
+namespace mbg {
 
 // Returns false when a tensor-core wait ran out (TC kernels only).
 template<typename T, int ALGO, int LEV, int C, int NT, bool UNIFORM, bool TC = false>
@@ -79,6 +265,8 @@ __device__ __forceinline__ bool tile_steps(
     const int32_t (&M)[C],
     const T* sh_coef,
     const tile_lists& tl,
+    const src_values<T>& sv,
+    tile_own<T> own,
     T* sh_a,
     T* sh_al,
     T* sh_b,
@@ -114,8 +302,6 @@ __device__ __forceinline__ bool tile_steps(
     const creg_t creg(sh_coef);
     bool sparse = false;
     if constexpr (REGCOEF && !DFD) sparse = cvr2_sparse(sh_coef);
-    const int nsrc = tl.overflow ? (int) (rd.src_end - rd.src_begin) : tl.nsrc;
-    const int nrec = tl.overflow ? (int) (rd.rec_end - rd.rec_begin) : tl.nrec;
     // Mirror walls are handled only on tiles of the non-uniform path (the
     // set-up marks a tile whose window holds a wall non-uniform): code that
     // touches H around the time loop, even off its hot path, costs the
@@ -146,6 +332,7 @@ __device__ __forceinline__ bool tile_steps(
     }
     for (int m = 0; m < nsteps; m++) {
         const uint64_t n = step0 + (uint64_t) m;
+        const uint32_t due = due_records(p, tl, own, m);
         // ---- E: needs H (hi, lo) of the right neighbour
         if (lane == 0) {
             sh_a[warp] = H[0];
@@ -176,26 +363,21 @@ __device__ __forceinline__ bool tile_steps(
             }
         }
         // ---- sources, after E and before H (solver_cpu_fdtd.tpp:245-255)
-        for (int s = 0; s < nsrc; s++) {
-            const src_desc sd = tl.overflow ? p.srcs[rd.src_begin + s] : tl.src[s];
-            const int64_t jj = (int64_t) sd.x_idx - l0;
-            if (jj >= 0 && jj < C) {
-                const double v = p.stab[sd.table_offset + n];
+        for_sources(p, rd, tl, sv, own, l0, m, nsteps, n, [&](int jj, int type, T vh, T vl) {
 #pragma unroll
-                for (int j = 0; j < C; j++) {
-                    if (j != jj || M[j] < 0) continue;
-                    if (sd.type == 0) {
-                        E[j] = (T) v;
-                        if constexpr (DF) El[j] = (T) (v - (double) E[j]);
-                    } else {
-                        if constexpr (DF)
-                            df_add(E[j], El[j], v);
-                        else
-                            E[j] += (T) v;
-                    }
+            for (int j = 0; j < C; j++) {
+                if (j != jj || M[j] < 0) continue;
+                if (type == 0) {
+                    E[j] = vh;
+                    if constexpr (DF) El[j] = vl;
+                } else {
+                    if constexpr (DF)
+                        df_add(E[j], El[j], vh, vl);
+                    else
+                        E[j] += vh;
                 }
             }
-        }
+        });
         // ---- H: needs E (hi, lo) of the left neighbour
         if (lane == 31) {
             sh_b[warp] = E[C - 1];
@@ -309,62 +491,62 @@ __device__ __forceinline__ bool tile_steps(
             }
         }
         // ---- recording (solver_cpu_fdtd.tpp:288-325)
-        if (p.record) {
-            for (int r = 0; r < nrec; r++) {
-                if (!tl.overflow && !tl.is_due(r, m)) continue;
-                const rec_desc rc = tl.overflow ? p.recs[rd.rec_begin + r] : tl.rec[r];
-                if (tl.overflow && rc.ratio != 1.0 && !hasto_record(rc.ratio, n)) continue;
-                const int64_t lo = max((int64_t) rc.pos, (int64_t) td.out_start);
-                const int64_t hi = min((int64_t) rc.pos + rc.cols, (int64_t) td.out_start + td.out_len);
-                if (l0 + C <= lo || l0 >= hi) continue;
-                const uint64_t row = rc.ratio == 1.0 ? n : (uint64_t) floor(rc.ratio * (double) n);
-                if (row >= rc.rows) continue;
+        auto field = [&](int jj, int type) {
+            T v = T(0);
 #pragma unroll
-                for (int j = 0; j < C; j++) {
-                    const int64_t l = l0 + j;
-                    if (l < lo || l >= hi) continue;
-                    const T ev = DF ? E[j] + El[j] : E[j];
-                    const T hv = DF ? H[j] + Hl[j] : H[j];
-                    T v = T(0);
-                    if constexpr (ALGO == 2) {
-                        switch (rc.type) {
-                        case 0: v = ev; break;
-                        case 1: v = P[j]; break;
-                        case 2: v = hv; break;
-                        case 4: v = DFD ? (R[j][1] - R[j][0]) + (Rl[j][1] - Rl[j][0]) : R[j][1] - R[j][0]; break;
-                        default: {
-                            // populations (3) and coherence parts (REC_COH_*):
-                            // an entry of the packed matrix (diagonal, then
-                            // the upper triangle as (re, im) pairs); constant
-                            // indices keep R in registers
-                            const uint32_t a = min(rc.row_idx, rc.col_idx);
-                            const uint32_t b = max(rc.row_idx, rc.col_idx);
-                            uint32_t idx = rc.type == 3 ? (a == b ? a : 0xffffffffu)
-                                                        : LEV + 2 * (b * (b - 1) / 2 + a) +
-                                                            (rc.type == REC_COH_IM ? 1 : 0);
+            for (int j = 0; j < C; j++)
+                if (j == jj)
+                    v = type == 0 ? (DF ? E[j] + El[j] : E[j]) : type == 1 ? P[j] : (DF ? H[j] + Hl[j] : H[j]);
+            return v;
+        };
+        for_records(p, rd, tl, own, due, m, n, field, [&](const rec_desc& rc, uint64_t row) {
+            const int64_t lo = max((int64_t) rc.pos, (int64_t) td.out_start);
+            const int64_t hi = min((int64_t) rc.pos + rc.cols, (int64_t) td.out_start + td.out_len);
 #pragma unroll
-                            for (int q = 0; q < LEV * LEV; q++)
-                                if (idx == (uint32_t) q) v = DFD ? R[j][q] + Rl[j][q] : R[j][q];
-                            if (rc.type == REC_COH_IM && rc.row_idx > rc.col_idx) v = -v;
-                            break;
-                        }
-                        }
-                    } else {
-                        constexpr int DDv = D > 0 ? D : 1;
-                        T u[DDv];
+            for (int j = 0; j < C; j++) {
+                const int64_t l = l0 + j;
+                if (l < lo || l >= hi) continue;
+                const T ev = DF ? E[j] + El[j] : E[j];
+                const T hv = DF ? H[j] + Hl[j] : H[j];
+                T v = T(0);
+                if constexpr (ALGO == 2) {
+                    switch (rc.type) {
+                    case 0: v = ev; break;
+                    case 1: v = P[j]; break;
+                    case 2: v = hv; break;
+                    case 4: v = DFD ? (R[j][1] - R[j][0]) + (Rl[j][1] - Rl[j][0]) : R[j][1] - R[j][0]; break;
+                    default: {
+                        // populations (3) and coherence parts (REC_COH_*):
+                        // an entry of the packed matrix (diagonal, then
+                        // the upper triangle as (re, im) pairs); constant
+                        // indices keep R in registers
+                        const uint32_t a = min(rc.row_idx, rc.col_idx);
+                        const uint32_t b = max(rc.row_idx, rc.col_idx);
+                        uint32_t idx = rc.type == 3 ? (a == b ? a : 0xffffffffu)
+                                                    : LEV + 2 * (b * (b - 1) / 2 + a) +
+                                                        (rc.type == REC_COH_IM ? 1 : 0);
 #pragma unroll
-                        for (int q = 0; q < DDv; q++) u[q] = DFD ? R[j][q] + Rl[j][q] : R[j][q];
-                        // the padded shared copy lacks the record rows, the
-                        // staged copy the coherence rows
-                        const T* rb = (PADC || rc.type >= REC_COH_RE) ? p.mc + (uint64_t) M[j] * p.mstride
-                                                                       : block(j);
-                        v = cvr_record_value<T, D>(rc, ev, hv, P[j], u, rb, LEV);
+                        for (int q = 0; q < LEV * LEV; q++)
+                            if (idx == (uint32_t) q) v = DFD ? R[j][q] + Rl[j][q] : R[j][q];
+                        if (rc.type == REC_COH_IM && rc.row_idx > rc.col_idx) v = -v;
+                        break;
                     }
-                    p.scratch[rc.offset + row * rc.cols + (uint64_t) (l - rc.pos)] = v;
-                    if (!isfinite(v)) atomicOr(p.status, STATUS_NONFINITE);
+                    }
+                } else {
+                    constexpr int DDv = D > 0 ? D : 1;
+                    T u[DDv];
+#pragma unroll
+                    for (int q = 0; q < DDv; q++) u[q] = DFD ? R[j][q] + Rl[j][q] : R[j][q];
+                    // the padded shared copy lacks the record rows, the
+                    // staged copy the coherence rows
+                    const T* rb = (PADC || rc.type >= REC_COH_RE) ? p.mc + (uint64_t) M[j] * p.mstride
+                                                                   : block(j);
+                    v = cvr_record_value<T, D>(rc, ev, hv, P[j], u, rb, LEV);
                 }
+                p.scratch[rc.offset + row * rc.cols + (uint64_t) (l - rc.pos)] = v;
+                if (!isfinite(v)) atomicOr(p.status, STATUS_NONFINITE);
             }
-        }
+        });
     }
     if (!UNIFORM && tl.wall) {
         // the point beyond the right end goes back to zero state (a bulk
@@ -434,6 +616,7 @@ __device__ __forceinline__ void step_body(const kparams<T>& p, uint32_t tile, ui
     constexpr bool DFD = DF && ALGO != 0;  // FP32 density state as float pairs
     __shared__ T sh_a[NW], sh_al[NW], sh_b[NW], sh_bl[NW];
     __shared__ tile_lists tl;
+    __shared__ src_values<T> sv;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T* sh_coef = reinterpret_cast<T*>(smem_raw);
 
@@ -485,6 +668,7 @@ __device__ __forceinline__ void step_body(const kparams<T>& p, uint32_t tile, ui
         tl.nsrc = ns;
         tl.nrec = nr;
         tl.overflow = of;
+        tl.staged = !of && ns * nsteps <= TILE_SRC_VALUES;
         // a mirror wall inside the window: point 0 or the point beyond the
         // right end (index n_x)
         tl.wall = (rd.k_left != 0.0 && w0 <= 0 && 0 < w1) ||
@@ -584,9 +768,11 @@ __device__ __forceinline__ void step_body(const kparams<T>& p, uint32_t tile, ui
         }
     }
     __syncthreads();
-    if (p.record && !tl.overflow && tl.nrec > 0) {  // the same in every thread
-        mark_due<NT>(tl, step0, nsteps);
+    tile_own<T> own{ 0u, -1, -1, 0u, nullptr };
+    if (tl.nsrc + tl.nrec > 0 || tl.overflow) {  // the same in every thread
+        prepare_lists<T, NT>(p, tl, sv, step0, nsteps);
         __syncthreads();
+        own = own_lists<T, C>(p, tl, td, l0, nsteps);
     }
 
     if constexpr (TC) {
@@ -609,21 +795,28 @@ __device__ __forceinline__ void step_body(const kparams<T>& p, uint32_t tile, ui
 
     if (uniform) {
         if constexpr (pair_path<T, ALGO, LEV, C, TC>()) {
-            // two points per instruction (pair_steps.cuh)
-            if (cvr2_sparse(sh_coef))
-                tile_steps_pair<C, NT, true>(p, td, rd, l0, nsteps, step0, E, H, P, R, Rl, M, sh_coef, tl, sh_a, sh_b);
+            // two points per instruction (pair_steps.cuh); tiles without
+            // sources and records in a loop that knows nothing of them
+            const bool sp = cvr2_sparse(sh_coef), lists = tl.nsrc + tl.nrec > 0 || tl.overflow;
+            auto run = [&](auto SP, auto LISTS) {
+                tile_steps_pair<C, NT, decltype(SP)::value, decltype(LISTS)::value>(
+                    p, td, rd, l0, nsteps, step0, E, H, P, R, Rl, M, sh_coef, tl, sv, own, sh_a, sh_b);
+            };
+            if (sp && !lists)
+                run(std::true_type{}, std::false_type{});
+            else if (sp)
+                run(std::true_type{}, std::true_type{});
             else
-                tile_steps_pair<C, NT, false>(p, td, rd, l0, nsteps, step0, E, H, P, R, Rl, M, sh_coef, tl, sh_a,
-                                              sh_b);
+                run(std::false_type{}, std::true_type{});
         } else {
             const bool ok = tile_steps<T, ALGO, LEV, C, NT, true, TC>(p, td, rd, l0, nsteps, step0, E, El, H, Hl,
-                                                                      P, R, Rl, M, sh_coef, tl, sh_a, sh_al,
-                                                                      sh_b, sh_bl, &tcc);
+                                                                      P, R, Rl, M, sh_coef, tl, sv, own, sh_a,
+                                                                      sh_al, sh_b, sh_bl, &tcc);
             if (!ok && threadIdx.x == 0) atomicOr(p.status, STATUS_TC_WAIT);
         }
     } else {
         tile_steps<T, ALGO, LEV, C, NT, false>(p, td, rd, l0, nsteps, step0, E, El, H, Hl, P, R, Rl, M,
-                                               sh_coef, tl, sh_a, sh_al, sh_b, sh_bl);
+                                               sh_coef, tl, sv, own, sh_a, sh_al, sh_b, sh_bl);
     }
     if constexpr (TC) {
         // every thread holds the same phase; the next tile of a persistent
