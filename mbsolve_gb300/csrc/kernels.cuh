@@ -121,21 +121,27 @@ __device__ __forceinline__ void rot_coeffs<float>(float x, float& s, float& s2)
 // chain of dependent operations or several, one lane or 32: measured), so
 // the count of FP64 instructions is the time of the FP64 kernels. Series in
 // Horner form by compile-time reciprocals (a division takes ten
-// instructions), as many terms as the range needs: for |x| < 2^-9 (the
-// field rotation of a step in the workloads here) the first omitted terms
-// are below 1e-20 of the result, for |x| < 1/4 below 1e-17; 8 and 18
-// instructions. With the 20 divisions of a recurrence before, a 2-level
+// instructions), as many terms as the range needs: for |x| < 2^-6 (fields up
+// to ten times the strongest of the presets) the first omitted terms are
+// below 2^-65 of the result, for |x| < 1/4 below 1e-17; 10 and 18
+// instructions. The range is read from the exponent bits: an FP64 compare
+// would be one more. With the 20 divisions of a recurrence before, a 2-level
 // point and step took 193 FP64 instructions; now about 30 (2-level preset,
-// 32,768 points: 1.98e9 -> 8.1e9 cell-updates/s; 6 levels, 65,536 points:
-// 9.5e7 -> 3.2e8, the unit's rate for the 1,225 products of a step).
+// 32,768 points, 10,000 steps: 165.6 -> 33.4 ms; 6 levels, 65,536 points: 9.5e7 ->
+// 3.2e8 cell-updates/s, the unit's rate for the 1,225 products of a step).
 template<>
 __device__ __forceinline__ void rot_coeffs<double>(double x, double& s, double& s2)
 {
     const double x2 = x * x;
-    if (fabs(x) < 0.001953125) {
-        s = fma(x * x2, fma(x2, 1.0 / 120.0, -1.0 / 6.0), x);
-        s2 = x2 * fma(x2, fma(x2, 1.0 / 720.0, -1.0 / 24.0), 0.5);
-    } else if (fabs(x) < 0.25) {
+    const int mag = __double2hiint(x) & 0x7fffffff;  // exponent and leading bits of |x|
+    if (mag < 0x3f900000) {                          // |x| < 2^-6
+        double t = fma(x2, -1.0 / 5040.0, 1.0 / 120.0);
+        t = fma(x2, t, -1.0 / 6.0);
+        s = fma(x * x2, t, x);
+        double u = fma(x2, -1.0 / 40320.0, 1.0 / 720.0);
+        u = fma(x2, u, -1.0 / 24.0);
+        s2 = x2 * fma(x2, u, 0.5);
+    } else if (mag < 0x3fd00000) {  // |x| < 1/4
         // sin x = x (1 - x^2/3! + ... + x^12/13!)
         double t = fma(x2, 1.0 / 6227020800.0, -1.0 / 39916800.0);
         t = fma(x2, t, 1.0 / 362880.0);
@@ -446,13 +452,17 @@ __device__ __forceinline__ void df_renorm(float& h, float& l)
 // (0, 1) plane, the free evolution couples 0 and 2 (precession) and relaxes
 // 1 on its own, and P reads 0 and 2. A uniform tile whose block has them
 // zero skips their products (a product with an exact zero changes no sum).
+// (Tested on the bits: see rot_coeffs<double>.)
+__device__ __forceinline__ bool is_zero(float v) { return (__float_as_uint(v) << 1) == 0u; }
+__device__ __forceinline__ bool is_zero(double v) { return ((unsigned long long) __double_as_longlong(v) << 1) == 0ull; }
+
 template<typename T>
 __device__ __forceinline__ bool cvr2_sparse(const T* cb)
 {
     const cvr_coef<T, 3> c{ cb };
-    return c.Bd(0, 1) == T(0) && c.Bd(1, 0) == T(0) && c.Bd(1, 2) == T(0) && c.Bd(2, 1) == T(0) &&
-        c.Bdl(0, 1) == T(0) && c.Bdl(1, 0) == T(0) && c.Bdl(1, 2) == T(0) && c.Bdl(2, 1) == T(0) &&
-        c.g(1) == T(0);
+    return is_zero(c.Bd(0, 1)) && is_zero(c.Bd(1, 0)) && is_zero(c.Bd(1, 2)) && is_zero(c.Bd(2, 1)) &&
+        is_zero(c.Bdl(0, 1)) && is_zero(c.Bdl(1, 0)) && is_zero(c.Bdl(1, 2)) && is_zero(c.Bdl(2, 1)) &&
+        is_zero(c.g(1));
 }
 
 // Coefficients of the 2-level update held in registers (uniform tiles).

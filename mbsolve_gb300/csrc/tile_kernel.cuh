@@ -300,8 +300,13 @@ __device__ __forceinline__ bool tile_steps(
     const bool qm_uniform = UNIFORM && sh_coef[pre::FD_HAS_QM] != T(0);
     using creg_t = typename std::conditional<REGCOEF, cvr_coef_reg<T, 3>, no_coef>::type;
     const creg_t creg(sh_coef);
-    bool sparse = false;
-    if constexpr (REGCOEF && !DFD) sparse = cvr2_sparse(sh_coef);
+    // FP64, 2 levels: points whose block has the zeros of cvr2_sparse
+    uint32_t sparse = 0u;
+    if constexpr (!DFD && ALGO == 1 && D == 3) {
+#pragma unroll
+        for (int j = 0; j < C; j++)
+            if (M[j] >= 0 && cvr2_sparse(block(j))) sparse |= 1u << j;
+    }
     // Mirror walls are handled only on tiles of the non-uniform path (the
     // set-up marks a tile whose window holds a wall non-uniform): code that
     // touches H around the time loop, even off its hot path, costs the
@@ -455,13 +460,13 @@ __device__ __forceinline__ bool tile_steps(
             for (int j = 0; j < C; j++) {
                 if (M[j] < 0) continue;
                 const T* cb = block(j);
-                if (UNIFORM ? !qm_uniform : cb[pre::FD_HAS_QM] == T(0)) continue;
+                if (UNIFORM ? !qm_uniform : is_zero(cb[pre::FD_HAS_QM])) continue;
                 const T e = DF ? E[j] + El[j] : E[j];
                 if constexpr (ALGO == 1) {
                     if constexpr (REGCOEF) {
                         if constexpr (DFD)
                             cvr_update_df<D>(R[j], Rl[j], e, P[j], creg);
-                        else if (sparse)
+                        else if ((sparse >> j) & 1u)
                             cvr_update<true>(R[j], e, P[j], creg);
                         else
                             cvr_update(R[j], e, P[j], creg);
@@ -478,10 +483,16 @@ __device__ __forceinline__ bool tile_steps(
                             cvr_update(R[j], e, P[j], cf);
                     } else {
                         cvr_coef<T, D> cf{ cb };
-                        if constexpr (DFD)
+                        if constexpr (DFD) {
                             cvr_update_df<D>(R[j], Rl[j], e, P[j], cf);
-                        else
+                        } else if constexpr (D == 3) {
+                            if ((sparse >> j) & 1u)
+                                cvr_update<true>(R[j], e, P[j], cf);
+                            else
+                                cvr_update(R[j], e, P[j], cf);
+                        } else {
                             cvr_update(R[j], e, P[j], cf);
+                        }
                     }
                 } else if constexpr (DFD) {
                     cayley_update_df<LEV>(R[j], Rl[j], e, P[j], cb);
