@@ -127,6 +127,10 @@ void launch_precompute(
     int* codes,
     cudaStream_t s);
 
+// Values of kernel_entry::staging: how a kernel holds its tile. POINT: the
+// kernels of runs of a single grid point (point_cayley.cuh).
+enum : int { STAGING_REGS = 0, STAGING_BULK = 1, STAGING_POINT = 2 };
+
 // Kernel registry: every instantiated (algo, levels, C, NT) launcher.
 template<typename T>
 using launch_fn = void (*)(const kparams<T>&, unsigned grid, size_t smem, cudaStream_t s);
@@ -140,7 +144,7 @@ template<typename T>
 struct kernel_entry {
     int algo, lev, C, NT;
     launch_fn<T> fn;
-    int staging;  // 0: tile state loaded into registers, 1: bulk-copy (TMA) staging
+    int staging;  // STAGING_*
     persist_fn<T> pfn;  // null where the shape has no persistent kernel
 };
 

@@ -65,6 +65,44 @@ struct src_values {
     T lo[sizeof(T) == 4 ? TILE_SRC_VALUES : 1];
 };
 
+// One thread: the sources inside the tile's window of `width` points (halo
+// included: the halo points must see them too) and the records inside its
+// output range.
+template<typename T>
+__device__ __forceinline__ void gather_lists(const kparams<T>& p, const tile_desc& td, const run_desc& rd, int64_t halo,
+                                             int64_t width, int nsteps, tile_lists& tl)
+{
+    const int64_t w0 = (int64_t) td.out_start - halo;
+    const int64_t w1 = w0 + width;
+    int ns = 0, nr = 0, of = 0;
+    for (uint32_t s = rd.src_begin; s < rd.src_end; s++) {
+        const src_desc sd = p.srcs[s];
+        if ((int64_t) sd.x_idx < w0 || (int64_t) sd.x_idx >= w1) continue;
+        if (ns < TILE_MAX_SRC)
+            tl.src[ns++] = sd;
+        else
+            of = 1;
+    }
+    for (uint32_t r = rd.rec_begin; r < rd.rec_end; r++) {
+        const rec_desc rc = p.recs[r];
+        const int64_t lo = max((int64_t) rc.pos, (int64_t) td.out_start);
+        const int64_t hi = min((int64_t) rc.pos + rc.cols, (int64_t) td.out_start + td.out_len);
+        if (lo >= hi) continue;
+        if (nr < TILE_MAX_REC)
+            tl.rec[nr++] = rc;
+        else
+            of = 1;
+    }
+    tl.nsrc = ns;
+    tl.nrec = nr;
+    tl.overflow = of;
+    tl.staged = !of && ns * nsteps <= TILE_SRC_VALUES;
+    // a mirror wall inside the window: point 0 or the point beyond the
+    // right end (index n_x)
+    tl.wall = (rd.k_left != 0.0 && w0 <= 0 && 0 < w1) ||
+        (rd.k_right != 0.0 && w0 <= (int64_t) rd.n_x && (int64_t) rd.n_x < w1);
+}
+
 // Fills the schedules and the sources' values; every thread calls it, a
 // barrier follows. The reference's predicate (hasto_record) runs once per
 // launch and step instead of once per step in every thread: about ten FP64
@@ -652,39 +690,7 @@ __device__ __forceinline__ void step_body(const kparams<T>& p, uint32_t tile, ui
     int nsteps = 0;
     if (step0 < rd.n_t) nsteps = (int) min((uint64_t) p.nsub, (uint64_t) rd.n_t - step0);
 
-    // sources inside the tile's window (halo included: the halo points
-    // must see them too) and records inside its output range
-    if (threadIdx.x == 0) {
-        const int64_t w0 = (int64_t) td.out_start - (int64_t) p.halo;
-        const int64_t w1 = w0 + (int64_t) NT * C;
-        int ns = 0, nr = 0, of = 0;
-        for (uint32_t s = rd.src_begin; s < rd.src_end; s++) {
-            const src_desc sd = p.srcs[s];
-            if ((int64_t) sd.x_idx < w0 || (int64_t) sd.x_idx >= w1) continue;
-            if (ns < TILE_MAX_SRC)
-                tl.src[ns++] = sd;
-            else
-                of = 1;
-        }
-        for (uint32_t r = rd.rec_begin; r < rd.rec_end; r++) {
-            const rec_desc rc = p.recs[r];
-            const int64_t lo = max((int64_t) rc.pos, (int64_t) td.out_start);
-            const int64_t hi = min((int64_t) rc.pos + rc.cols, (int64_t) td.out_start + td.out_len);
-            if (lo >= hi) continue;
-            if (nr < TILE_MAX_REC)
-                tl.rec[nr++] = rc;
-            else
-                of = 1;
-        }
-        tl.nsrc = ns;
-        tl.nrec = nr;
-        tl.overflow = of;
-        tl.staged = !of && ns * nsteps <= TILE_SRC_VALUES;
-        // a mirror wall inside the window: point 0 or the point beyond the
-        // right end (index n_x)
-        tl.wall = (rd.k_left != 0.0 && w0 <= 0 && 0 < w1) ||
-            (rd.k_right != 0.0 && w0 <= (int64_t) rd.n_x && (int64_t) rd.n_x < w1);
-    }
+    if (threadIdx.x == 0) gather_lists(p, td, rd, (int64_t) p.halo, (int64_t) NT * C, nsteps, tl);
 
     T E[C], El[C], H[C], Hl[C], P[C];
     T R[C][DD];
