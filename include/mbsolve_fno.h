@@ -200,6 +200,40 @@ int mbg_fno_envelope(const double* e, int32_t runs, int32_t rows,
                      int32_t nout, double tout0, double dtout, float* out,
                      void* stream);
 
+/* A sequence of the calls above, issued on one stream in order by one call
+ * (a layer's or a training step's launches take the host longer to prepare
+ * one by one than the GPU to run). The fields each kind reads:
+ *   GEMM, LAYER    desc (mbg_gemm_desc, mbg_fno_layer_desc)
+ *   MODE_BLOCKS    in[0] wr, in[1] wi, i[0] modes, i[1] width, out[0] blk
+ *   CAST           in[0] x, n[0] count, out[0] y
+ *   IMAGE          in[0] x, i[0..4] batch, rows, cols, R, K, n[0] ld,
+ *                  n[1] zs, out[0] img
+ *   COLSUM         in[0] x, n[0] rows, i[0] cols, n[1] row stride, out[0]
+ *   MSE            in[0] y, in[1] t, n[0] count, out[0] grad, out[1] loss
+ *   ZERO           out[0], n[0] bytes set to zero
+ * Returns the first call's error; the calls after it are not issued. */
+enum {
+    MBG_OP_GEMM = 0,
+    MBG_OP_LAYER = 1,
+    MBG_OP_MODE_BLOCKS = 2,
+    MBG_OP_CAST = 3,
+    MBG_OP_IMAGE = 4,
+    MBG_OP_COLSUM = 5,
+    MBG_OP_MSE = 6,
+    MBG_OP_ZERO = 7
+};
+
+typedef struct mbg_fno_op {
+    int32_t kind;
+    int32_t i[5];
+    int64_t n[2];
+    const void* in[2];
+    void* out[2];
+    const void* desc;
+} mbg_fno_op;
+
+int mbg_fno_run(const mbg_fno_op* ops, int32_t count, void* stream);
+
 /* Kernel-side status since the last call (bit 0: a tensor-core wait ran
  * out; bit 1: TMEM allocation refused); cleared by the call. */
 int mbg_fno_status(uint32_t* status);

@@ -102,6 +102,7 @@ def load():
                                i32, vp]
     L.mbg_fno_envelope.argtypes = [vp, i32, i32, i64, f64, f64, f64, i32,
                                    f64, f64, vp, vp]
+    L.mbg_fno_run.argtypes = [P(T.mbg_fno_op), i32, vp]
     L.mbg_fno_status.argtypes = [P(C.c_uint32)]
     _lib = L
     return L

@@ -209,3 +209,18 @@ class mbg_fno_layer_desc(C.Structure):
         ("Q1", C.c_void_p), ("bq1", C.c_void_p), ("q2", C.c_void_p),
         ("bq2", C.c_void_p), ("y", C.c_void_p),
     ]
+
+
+(MBG_OP_GEMM, MBG_OP_LAYER, MBG_OP_MODE_BLOCKS, MBG_OP_CAST, MBG_OP_IMAGE,
+ MBG_OP_COLSUM, MBG_OP_MSE, MBG_OP_ZERO) = range(8)
+
+
+class mbg_fno_op(C.Structure):
+    _fields_ = [
+        ("kind", C.c_int32),
+        ("i", C.c_int32 * 5),
+        ("n", C.c_int64 * 2),
+        ("in_", C.c_void_p * 2),
+        ("out", C.c_void_p * 2),
+        ("desc", C.c_void_p),
+    ]

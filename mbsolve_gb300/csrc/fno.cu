@@ -1036,6 +1036,42 @@ int mbg_fno_envelope(const double* e, int32_t runs, int32_t rows, int64_t run_st
     });
 }
 
+int mbg_fno_run(const mbg_fno_op* ops, int32_t count, void* stream)
+{
+    int rc = guard([&] { require(count >= 0 && (ops || count == 0), "run: bad arguments"); });
+    for (int32_t k = 0; k < count && rc == MBG_OK; k++) {
+        const mbg_fno_op& o = ops[k];
+        const float* x = static_cast<const float*>(o.in[0]);
+        const float* y = static_cast<const float*>(o.in[1]);
+        switch (o.kind) {
+        case MBG_OP_GEMM: rc = mbg_fno_gemm(static_cast<const mbg_gemm_desc*>(o.desc), stream); break;
+        case MBG_OP_LAYER:
+            rc = mbg_fno_spectral_layer(static_cast<const mbg_fno_layer_desc*>(o.desc), stream);
+            break;
+        case MBG_OP_MODE_BLOCKS: rc = mbg_fno_mode_blocks(x, y, o.i[0], o.i[1], o.out[0], stream); break;
+        case MBG_OP_CAST: rc = mbg_fno_cast_bf16(x, o.out[0], o.n[0], stream); break;
+        case MBG_OP_IMAGE:
+            rc = mbg_fno_image_bf16(x, o.i[0], o.i[1], o.i[2], o.n[0], o.n[1], o.i[3], o.i[4], o.out[0], stream);
+            break;
+        case MBG_OP_COLSUM:
+            rc = mbg_fno_colsum(x, o.n[0], o.i[0], o.n[1], static_cast<float*>(o.out[0]), stream);
+            break;
+        case MBG_OP_MSE:
+            rc = mbg_fno_mse(x, y, o.n[0], static_cast<float*>(o.out[0]), static_cast<float*>(o.out[1]), stream);
+            break;
+        case MBG_OP_ZERO:
+            rc = guard([&] {
+                require(o.out[0] && o.n[0] > 0, "zero: bad arguments");
+                if (cudaMemsetAsync(o.out[0], 0, (size_t) o.n[0], (cudaStream_t) stream) != cudaSuccess)
+                    check_launch("memset");
+            });
+            break;
+        default: rc = guard([] { require(false, "run: unknown operation"); });
+        }
+    }
+    return rc;
+}
+
 int mbg_fno_status(uint32_t* status)
 {
     return guard([&] {

@@ -112,11 +112,36 @@ class FNO:
                                 device=self.dev) for _ in range(sh.L)]
         self._bufs = {}
         self._ibufs = {}
-        self._blk_valid = False
+        self._progs = {}
+        self._blk_valid = False   # blk: BF16 mode blocks of the weights
+        self._dense_valid = False  # _wb, _img: what infer() reads besides
         self._wb = {}   # BF16 copies of the dense weights (inference)
         self._img = {}  # BF16 tile images for the fused layer kernel
 
+    def __getstate__(self):
+        # a copy lays its own programs out: they hold device addresses
+        d = self.__dict__.copy()
+        d["_progs"] = {}
+        return d
+
     # ------------------------------------------------------------ helpers
+    def _issue(self, key, calls, **inputs):
+        """The kernel calls of calls(**inputs): on a GPU laid out on the
+        first use of `key` (K.Program) and issued by one native call. Every
+        other tensor they touch belongs to this object and stays in place."""
+        if self.dev.type != "cuda":
+            calls(**inputs)
+            return
+        prog = self._progs.get(key)
+        if prog is None:
+            prog = K.Program()
+            for name, t in inputs.items():
+                prog.input(name, t)
+            with prog:
+                calls(**inputs)
+            self._progs[key] = prog
+        prog.run(**inputs)
+
     def _views(self, flat):
         out, o = {}, 0
         for name, shape in self.sh.param_spec():
@@ -127,7 +152,7 @@ class FNO:
 
     def load_params(self, theta):
         self.theta.copy_(torch.as_tensor(theta, dtype=torch.float32))
-        self._blk_valid = False
+        self._blk_valid = self._dense_valid = False
 
     def _buffers(self, B):
         if B in self._bufs:
@@ -153,10 +178,24 @@ class FNO:
         self._bufs[B] = b
         return b
 
+    def _weights(self, infer):
+        """Brings the BF16 forms of the weights up to date: the mode blocks,
+        and what only infer() reads."""
+        if not self._blk_valid:
+            self._issue("blk", self._mode_blocks)
+            self._blk_valid = True
+        if infer and not self._dense_valid:
+            if self.fused_ok() and "G" not in self._img:
+                self._basis_images()
+            self._issue("dense", self._dense_weights)
+            self._dense_valid = True
+
     def _mode_blocks(self):
         for l in range(self.sh.L):
             K.mode_blocks(self.p["wr%d" % l].view(self.sh.Mo, self.sh.W, self.sh.W),
                           self.p["wi%d" % l], self.blk[l])
+
+    def _dense_weights(self):
         # BF16 copies of the dense weights for infer() (the same rounding the
         # products apply to the FP32 weights when they load them)
         for name in ["W%d" % l for l in range(self.sh.L)] + ["Q1", "q2"]:
@@ -167,7 +206,6 @@ class FNO:
             K.cast_bf16(self.p[name], w)
         if self.fused_ok():
             self._layer_images()
-        self._blk_valid = True
 
     @staticmethod
     def _split(rows):
@@ -189,18 +227,24 @@ class FNO:
         if tuple(X.shape) != (B, S, Fi) or X.dtype != torch.float32:
             raise ValueError("X must be FP32 [B, %d, %d]" % (S, Fi))
         X = X.contiguous()
+        self._weights(False)
+        self._X = X
+        self._issue(("forward", B), self._forward_calls, X=X)
+        return self._buffers(B)["y"].view(B, S)
+
+    def _forward_calls(self, X):
+        sh = self.sh
+        S, W, Mo, L, Fi, Hq = sh.S, sh.W, sh.Mo, sh.L, sh.F, sh.Hq
+        B = X.shape[0]
         b = self._buffers(B)
         p = self.p
-        if not self._blk_valid:
-            self._mode_blocks()
-        self._X = X
         # lifting: v0 = X P^T + bp
         K.gemm(B * S, W, [Seg(X, 0, Fi, 1, 0, p["P"], 0, Fi, 1, 0, Fi)],
                b["v"][0], 0, W, 1, bias=p["bp"])
         for l in range(L):
             v, vh = b["v"][l], b["Vh"][l]
             # truncated DFT: Vh[b, m', c] = sum_s F[m', s] v[b, s, c]
-            vh.zero_()
+            K.zero(vh)
             K.gemm(2 * Mo, W, [Seg(self.F, 0, S, 1, 0, v, 0, 1, W, S * W, S)],
                    vh, 0, W, 1, 2 * Mo * W, batch=B,
                    mode=T.MBG_GEMM_ATOMIC, split_k=self.DFT_SPLIT)
@@ -224,7 +268,6 @@ class FNO:
                b["h"], 0, Hq, 1, bias=p["bq1"], act=T.MBG_ACT_GELU, pre=b["ph"])
         K.gemm(B * S, 1, [Seg(b["h"], 0, Hq, 1, 0, p["q2"], 0, 0, 1, 0, Hq)],
                b["y"], 0, 1, 1, bias=p["bq2"])
-        return b["y"].view(B, S)
 
     def _ibuffers(self, B):
         if B in self._ibufs:
@@ -250,21 +293,26 @@ class FNO:
         return (sh.S % 128 == 0 and sh.W <= 64 and 2 * sh.Mo <= 64
                 and sh.Hq <= 128 and sh.F <= 16)
 
-    def _layer_images(self):
-        """BF16 tile images for the fused layer kernel: the DFT bases (once)
-        and the dense weights (after every parameter change)."""
-        sh = self.sh
-        S, W, Mo, Hq = sh.S, sh.W, sh.Mo, sh.Hq
+    def _basis_images(self):
+        """BF16 tile images of the DFT bases for the fused layer kernel."""
+        S, Mo = self.sh.S, self.sh.Mo
         T, b16, d = S // 128, torch.bfloat16, self.dev
         im = self._img
-        if "G" not in im:
-            F, G = dft_bases(S, Mo)
-            F32 = torch.tensor(F, dtype=torch.float32, device=d)
-            G32 = torch.tensor(G, dtype=torch.float32, device=d)
-            im["G"] = torch.empty(T * 8192, dtype=b16, device=d)
-            im["F"] = torch.empty(T * 8192, dtype=b16, device=d)
-            K.image_bf16(G32, T, 128, 2 * Mo, 2 * Mo, 128 * 2 * Mo, 128, 64, im["G"])
-            K.image_bf16(F32, T, 2 * Mo, 128, S, 128, 64, 128, im["F"])
+        F, G = dft_bases(S, Mo)
+        F32 = torch.tensor(F, dtype=torch.float32, device=d)
+        G32 = torch.tensor(G, dtype=torch.float32, device=d)
+        im["G"] = torch.empty(T * 8192, dtype=b16, device=d)
+        im["F"] = torch.empty(T * 8192, dtype=b16, device=d)
+        K.image_bf16(G32, T, 128, 2 * Mo, 2 * Mo, 128 * 2 * Mo, 128, 64, im["G"])
+        K.image_bf16(F32, T, 2 * Mo, 128, S, 128, 64, 128, im["F"])
+
+    def _layer_images(self):
+        """BF16 tile images of the dense weights for the fused layer kernel
+        (after every parameter change)."""
+        sh = self.sh
+        W, Hq = sh.W, sh.Hq
+        b16, d = torch.bfloat16, self.dev
+        im = self._img
         for l in range(sh.L):
             name = "W%d" % l
             if name not in im:
@@ -310,13 +358,20 @@ class FNO:
         B = X.shape[0]
         if tuple(X.shape) != (B, S, Fi) or X.dtype != torch.float32:
             raise ValueError("X must be FP32 [B, %d, %d]" % (S, Fi))
-        if not self.fused_ok():
-            return self._infer_products(X)
         X = X.contiguous()
+        self._weights(True)
+        if not self.fused_ok():
+            self._issue(("infer", B), self._infer_products, X=X)
+            return self._ibuffers(B)["y"].view(B, S)
+        self._issue(("infer", B), self._infer_calls, X=X)
+        return self._fbuffers(B)["y"].view(B, S)
+
+    def _infer_calls(self, X):
+        sh = self.sh
+        S, W, Mo, L, Fi, Hq = sh.S, sh.W, sh.Mo, sh.L, sh.F, sh.Hq
+        B = X.shape[0]
         b = self._fbuffers(B)
         p = self.p
-        if not self._blk_valid:
-            self._mode_blocks()
         im = self._img
         vhT, Y = b["VhT"], b["Y"]
         K.spectral_layer(T.MBG_LAYER_LIFT, T.MBG_ACT_NONE, B, S, W, Mo, Fi=Fi,
@@ -346,7 +401,6 @@ class FNO:
                                  Wl=im["W%d" % l], bias=p["bw%d" % l],
                                  Q1=im["Q1"], bq1=p["bq1"], q2=p["q2"],
                                  bq2=p["bq2"], y=b["y"])
-        return b["y"].view(B, S)
 
     def _infer_products(self, X):
         """infer() for sizes the fused layer kernel does not take, as
@@ -360,16 +414,13 @@ class FNO:
         [B, 2 Mo, W] for the mixing; BF16 copies of the dense weights. The
         truncated DFT runs without split-K (K = S per sample); the output
         layer is folded into the hidden projection's epilogue; no
-        pre-activations are stored. X: FP32 [B, S, F]; returns
-        y [B, S] (a view of an internal buffer)."""
+        pre-activations are stored. X: FP32 [B, S, F]; the outputs go to
+        the batch's buffer "y"."""
         sh = self.sh
         S, W, Mo, L, Fi, Hq = sh.S, sh.W, sh.Mo, sh.L, sh.F, sh.Hq
         B = X.shape[0]
-        X = X.contiguous()
         b = self._ibuffers(B)
         p = self.p
-        if not self._blk_valid:
-            self._mode_blocks()
         wb = self._wb
         # lifting, per sample: v0[b] = X[b] P^T + bp, also as vT0[b] [W, S]
         K.gemm(S, W, [Seg(X, 0, Fi, 1, S * Fi, p["P"], 0, Fi, 1, 0, Fi)],
@@ -408,30 +459,33 @@ class FNO:
             cur = nxt
         # projection: y = q2 . GELU(v Q1^T + bq1) + bq2, the second product
         # folded into the first one's epilogue (no hidden activation stored)
-        b["y"].zero_()
+        K.zero(b["y"])
         K.gemm(B * S, Hq, [Seg(b["v"][cur], 0, W, 1, 0, wb["Q1"], 0, W, 1, 0, W)],
                b["y"], 0, 1, 0, bias=p["bq1"], act=T.MBG_ACT_GELU,
                rowdot=p["q2"], rowdot_bias=p["bq2"])
-        return b["y"].view(B, S)
 
     # ------------------------------------------------------------ backward
     def backward(self, dy=None):
         """Gradient of the loss into self.grad (zeroed first). dy: FP32
         [B, S] gradient of the loss w.r.t. the last forward's output, or
         None when loss() already wrote it."""
-        sh = self.sh
-        S, W, Mo, L, Fi, Hq = sh.S, sh.W, sh.Mo, sh.L, sh.F, sh.Hq
         X = self._X
         B = X.shape[0]
         if B % 8:
             raise ValueError("backward needs a batch that is a multiple of 8")
+        if dy is not None:
+            self._buffers(B)["dy"].copy_(dy.reshape(-1))
+        self._issue(("backward", B), self._backward_calls, X=X)
+
+    def _backward_calls(self, X):
+        sh = self.sh
+        S, W, Mo, L, Fi, Hq = sh.S, sh.W, sh.Mo, sh.L, sh.F, sh.Hq
+        B = X.shape[0]
         b = self._buffers(B)
         p, g = self.p, self.g
-        if dy is not None:
-            b["dy"].copy_(dy.reshape(-1))
         dyb = b["dy"]
         R = B * S
-        self.grad.zero_()
+        K.zero(self.grad)
         ATOM = T.MBG_GEMM_ATOMIC
         # output layer
         K.gemm(Hq, 1, [Seg(b["h"], 0, 1, Hq, 0, dyb, 0, 0, 1, 0, R)],
@@ -452,7 +506,7 @@ class FNO:
                    g["W%d" % l], 0, W, 1, mode=ATOM, split_k=self._split(R))
             K.colsum(dpre, R, W, W, g["bw%d" % l])
             # dY[b, m', o] = sum_s G[s, m'] dpre[b, s, o]
-            b["dY"].zero_()
+            K.zero(b["dY"])
             K.gemm(2 * Mo, W, [Seg(self.G, 0, 1, 2 * Mo, 0, dpre, 0, 1, W, S * W, S)],
                    b["dY"], 0, W, 1, 2 * Mo * W, batch=B,
                    mode=T.MBG_GEMM_ATOMIC, split_k=self.DFT_SPLIT)
@@ -496,15 +550,19 @@ class FNO:
         one-element CUDA tensor (no synchronisation)."""
         B = self._X.shape[0]
         b = self._buffers(B)
-        b["loss"].zero_()
-        K.mse(b["y"], target.reshape(-1), b["dy"], b["loss"])
+
+        def calls(target):
+            K.zero(b["loss"])
+            K.mse(b["y"], target, b["dy"], b["loss"])
+        t = target.reshape(-1)
+        self._issue(("loss", B, t.numel(), t.dtype, t.device), calls, target=t)
         return b["loss"]
 
     def adam(self, lr=1e-3, beta1=0.9, beta2=0.999, eps=1e-8, weight_decay=0.0):
         self.step_count += 1
         K.adam(self.theta, self.grad, self.m1, self.m2, lr, beta1, beta2, eps,
                weight_decay, self.step_count)
-        self._blk_valid = False
+        self._blk_valid = self._dense_valid = False
 
     def train_step(self, X, target, lr=1e-3, weight_decay=0.0):
         self.forward(X)

@@ -6,6 +6,7 @@ on the host that every element the kernel will touch lies inside its
 tensor, so a wrong stride raises here instead of reading out of bounds.
 """
 import ctypes as C
+import threading
 
 import torch
 
@@ -25,6 +26,90 @@ def _stream():
 
 def _ptr(t, off=0):
     return C.c_void_p(t.data_ptr() + int(off) * t.element_size())
+
+
+class Program:
+    """A fixed sequence of this module's calls, checked and laid out once
+    (``with Program() as p: ...``: calls inside are recorded, not issued) and
+    then issued by one native call (run()): preparing them one by one took
+    the host 24 us a call, longer than most of their kernels run.
+
+    The tensors of the recorded calls must outlive the program and stay where
+    they are, except those given to input(), which stand for the tensor
+    passed to run() under that name: same size, dtype and device, contiguous.
+    """
+
+    _local = threading.local()
+
+    def __init__(self):
+        self._ops, self._keep, self._inputs, self._patch = [], [], {}, []
+        self._array = None
+
+    def input(self, name, t):
+        self._inputs[name] = t
+        return t
+
+    def __enter__(self):
+        if getattr(Program._local, "now", None) is not None:
+            raise RuntimeError("a program is being recorded already")
+        Program._local.now = self
+        return self
+
+    def __exit__(self, kind, value, tb):
+        Program._local.now = None
+        if kind is None:
+            # an input is known by what run() checks; the tensor is not kept
+            self._keep = [t for t in self._keep
+                          if not any(t is u for u in self._inputs.values())]
+            self._inputs = {name: (t.shape, t.dtype, t.device)
+                            for name, t in self._inputs.items()}
+            self._array = (T.mbg_fno_op * len(self._ops))(*self._ops)
+            # descriptor fields that hold an input's address; the operations
+            # were copied into the array
+            self._patch = [(name, self._array[o[1]] if isinstance(o, tuple) else o, f, off)
+                           for name, o, f, off in self._patch]
+
+    def _add(self, kind, desc=None, i=(), n=(), ins=(), outs=()):
+        """ins, outs: tensors; desc: a descriptor structure."""
+        op = T.mbg_fno_op()
+        op.kind = kind
+        if desc is not None:
+            op.desc = C.addressof(desc)
+            self._keep.append(desc)
+        for k, v in enumerate(i):
+            op.i[k] = int(v)
+        for k, v in enumerate(n):
+            op.n[k] = int(v)
+        for k, t in enumerate(ins):
+            op.in_[k] = t.data_ptr()
+            self._note(t, (self, len(self._ops)), ("in_", k), 0)
+        for k, t in enumerate(outs):
+            op.out[k] = t.data_ptr()
+        self._keep.extend(list(ins) + list(outs))
+        self._ops.append(op)
+
+    def _note(self, t, where, field, off):
+        for name, u in self._inputs.items():
+            if t is u:
+                self._patch.append((name, where, field, off))
+
+    def run(self, **inputs):
+        for name, t in inputs.items():
+            want = self._inputs[name]
+            if (t.shape, t.dtype, t.device) != want or not t.is_contiguous():
+                raise ValueError("%s: need a contiguous tensor of %s, %s, %s"
+                                 % ((name,) + want))
+        for name, where, (attr, k), off in self._patch:
+            a = inputs[name].data_ptr() + off
+            if k is None:
+                setattr(where, attr, a)
+            else:
+                getattr(where, attr)[k] = a
+        _native.check(_lib().mbg_fno_run(self._array, len(self._ops), _stream()))
+
+
+def _recording():
+    return getattr(Program._local, "now", None)
 
 
 def _check_span(t, off, extents_strides, what):
@@ -114,6 +199,15 @@ def gemm(m, n, segs, c, c_off, c_sm, c_sn, c_sz=0, batch=1,
         d.rowdot = _ptr(rowdot)
         if rowdot_bias is not None:
             d.rowdot_bias = _ptr(rowdot_bias)
+    rec = _recording()
+    if rec is not None:
+        for i, s in enumerate(segs):
+            rec._note(s.a, d.seg[i], ("a", None), int(s.a_off) * s.a.element_size())
+            rec._note(s.b, d.seg[i], ("b", None), int(s.b_off) * s.b.element_size())
+        rec._keep.extend([t for s in segs for t in (s.a, s.b)] +
+                         [c, bias, pre, gate, c2, rowdot, rowdot_bias])
+        rec._add(T.MBG_OP_GEMM, d)
+        return
     _native.check(_lib().mbg_fno_gemm(C.byref(d), _stream()))
 
 
@@ -160,6 +254,13 @@ def spectral_layer(mode, act, batch, S, W, Mo, Fi=0, Hq=0, X=None, P=None,
         setattr(d, name, _ptr(t))
     d.mode, d.act, d.batch = int(mode), int(act), B
     d.S, d.W, d.Mo, d.Fi, d.Hq = int(S), int(W), int(Mo), int(Fi), int(Hq)
+    rec = _recording()
+    if rec is not None:
+        for name, (t, _, _) in need.items():
+            rec._note(t, d, (name, None), 0)
+            rec._keep.append(t)
+        rec._add(T.MBG_OP_LAYER, d)
+        return
     _native.check(_lib().mbg_fno_spectral_layer(C.byref(d), _stream()))
 
 
@@ -167,6 +268,10 @@ def mode_blocks(wr, wi, blk):
     modes, width = wr.shape[0], wr.shape[1]
     if blk.dtype != torch.bfloat16 or blk.numel() < modes * 4 * width * width:
         raise ValueError("mode_blocks: BF16 output of modes x 2w x 2w")
+    rec = _recording()
+    if rec is not None:
+        rec._add(T.MBG_OP_MODE_BLOCKS, i=(modes, width), ins=(wr, wi), outs=(blk,))
+        return
     _native.check(_lib().mbg_fno_mode_blocks(
         _ptr(wr), _ptr(wi), modes, width, _ptr(blk), _stream()))
 
@@ -174,6 +279,10 @@ def mode_blocks(wr, wi, blk):
 def cast_bf16(x, y):
     if x.numel() != y.numel() or y.dtype != torch.bfloat16:
         raise ValueError("cast_bf16: sizes or dtype")
+    rec = _recording()
+    if rec is not None:
+        rec._add(T.MBG_OP_CAST, n=(x.numel(),), ins=(x,), outs=(y,))
+        return
     _native.check(_lib().mbg_fno_cast_bf16(_ptr(x), _ptr(y), x.numel(),
                                            _stream()))
 
@@ -186,6 +295,11 @@ def image_bf16(x, batch, rows, cols, ld, zs, R, K, img):
     _check_span(x, 0, [(batch, zs), (rows, ld), (cols, 1)], "image_bf16 x")
     if img.numel() < batch * R * K or not img.is_contiguous():
         raise ValueError("image_bf16: image too small")
+    rec = _recording()
+    if rec is not None:
+        rec._add(T.MBG_OP_IMAGE, i=(batch, rows, cols, R, K), n=(ld, zs),
+                 ins=(x,), outs=(img,))
+        return
     _native.check(_lib().mbg_fno_image_bf16(_ptr(x), batch, rows, cols, ld,
                                             zs, R, K, _ptr(img), _stream()))
 
@@ -194,6 +308,11 @@ def colsum(x, rows, cols, row_stride, out):
     _check_span(x, 0, [(rows, row_stride), (cols, 1)], "colsum x")
     if out.numel() < cols:
         raise ValueError("colsum: out too small")
+    rec = _recording()
+    if rec is not None:
+        rec._add(T.MBG_OP_COLSUM, i=(cols,), n=(rows, row_stride), ins=(x,),
+                 outs=(out,))
+        return
     _native.check(_lib().mbg_fno_colsum(_ptr(x), rows, cols, row_stride,
                                         _ptr(out), _stream()))
 
@@ -202,8 +321,21 @@ def mse(y, t, grad, loss):
     n = y.numel()
     if t.numel() != n or grad.numel() != n or loss.numel() < 1:
         raise ValueError("mse: sizes")
+    rec = _recording()
+    if rec is not None:
+        rec._add(T.MBG_OP_MSE, n=(n,), ins=(y, t), outs=(grad, loss))
+        return
     _native.check(_lib().mbg_fno_mse(_ptr(y), _ptr(t), n, _ptr(grad),
                                      _ptr(loss), _stream()))
+
+
+def zero(t):
+    """All bytes of a contiguous tensor to zero."""
+    rec = _recording()
+    if rec is not None:
+        rec._add(T.MBG_OP_ZERO, n=(t.numel() * t.element_size(),), outs=(t,))
+        return
+    t.zero_()
 
 
 def adam(w, g, m, v, lr, beta1, beta2, eps, weight_decay, step):
