@@ -30,19 +30,24 @@ void launch_step_bulk(const kparams<float>& p, unsigned grid, size_t smem, cudaS
     step_kernel_bulk<C, NT><<<grid, NT, need, s>>>(p);
 }
 
-// FP32 coherence-vector kernels for 4-6 levels with the density products
-// of uniform tiles on the tensor cores (128 threads, one point each).
-template<int LEV>
-void launch_step_tc(const kparams<float>& p, unsigned grid, size_t smem, cudaStream_t s)
+// FP32 kernels for 4-6 levels with the density products of uniform tiles on
+// the tensor cores (128 threads, one point each): staged coefficients, then
+// the operands.
+template<int ALGO, int LEV>
+size_t tc_smem()
 {
-    constexpr int D = LEV * LEV - 1;
-    const size_t need = ((tc::coef_small<D>::len * sizeof(float) + 127) & ~(size_t) 127) + 128 +
-        tc::shape<D>::BYTES;
-    if (smem < need) smem = need;
+    return ((tc_coef_len<ALGO, LEV>() * sizeof(float) + 127) & ~(size_t) 127) + 128 +
+        tc::shape<density_len<ALGO, LEV>::value>::BYTES;
+}
+
+template<int ALGO, int LEV>
+void launch_step_tc(const kparams<float>& p, unsigned grid, size_t, cudaStream_t s)
+{
+    const size_t smem = tc_smem<ALGO, LEV>();
     static const cudaError_t attr = cudaFuncSetAttribute(
-        step_kernel_tc<LEV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) need);
+        step_kernel_tc<ALGO, LEV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
     (void) attr;
-    step_kernel_tc<LEV><<<grid, tc::M, smem, s>>>(p);
+    step_kernel_tc<ALGO, LEV><<<grid, tc::M, smem, s>>>(p);
 }
 
 // Persistent kernels: as many CTAs as fit the SMs at once. They need not
@@ -102,15 +107,12 @@ unsigned launch_persist(const kparams<T>& p, const persist_params& q, size_t sme
     return persist_launch(step_kernel_persist<T, ALGO, LEV, C, NT>, NT, smem, q.levels * q.n_tiles, s, p, q);
 }
 
-template<int LEV>
-unsigned launch_persist_tc(const kparams<float>& p, const persist_params& q, size_t smem, cudaStream_t s)
+template<int ALGO, int LEV>
+unsigned launch_persist_tc(const kparams<float>& p, const persist_params& q, size_t, cudaStream_t s)
 {
-    constexpr int D = LEV * LEV - 1;
-    const size_t need = ((tc::coef_small<D>::len * sizeof(float) + 127) & ~(size_t) 127) + 128 +
-        tc::shape<D>::BYTES;
-    if (smem < need) smem = need;
-    auto k = step_kernel_persist_tc<LEV>;
-    static const cudaError_t attr = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) need);
+    const size_t smem = tc_smem<ALGO, LEV>();
+    auto k = step_kernel_persist_tc<ALGO, LEV>;
+    static const cudaError_t attr = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
     (void) attr;
     return persist_launch(k, tc::M, smem, q.levels * q.n_tiles, s, p, q);
 }
@@ -118,23 +120,18 @@ unsigned launch_persist_tc(const kparams<float>& p, const persist_params& q, siz
 }  // namespace mbg
 
 // with a persistent kernel as well
-#define MBG_REG_CVR_TC_P(LEV)                                                      \
+#define MBG_REG_TC_P(ALGO, LEV)                                                    \
     static const bool MBG_CAT(mbg_reg_, __LINE__) = ::mbg::register_kernel<float>( \
-        ::mbg::ALGO_CVR, LEV, 1, ::mbg::tc::M, &::mbg::launch_step_tc<LEV>, 0,      \
-        &::mbg::launch_persist_tc<LEV>);
-// only the persistent kernel of a shape registered elsewhere (a
-// translation unit of its own, so that no kernel is compiled twice)
-#define MBG_REG_CAY_PONLY(T, LEV, C, NT)                                       \
+        ::mbg::ALGO, LEV, 1, ::mbg::tc::M, &::mbg::launch_step_tc<::mbg::ALGO, LEV>, 0, \
+        &::mbg::launch_persist_tc<::mbg::ALGO, LEV>);
+#define MBG_REG_CAY_P(T, LEV, C, NT)                                           \
     static const bool MBG_CAT(mbg_reg_, __LINE__) = ::mbg::register_kernel<T>( \
-        ::mbg::ALGO_CAYLEY, LEV, C, NT, nullptr, 0, &::mbg::launch_persist<T, 2, LEV, C, NT>);
+        ::mbg::ALGO_CAYLEY, LEV, C, NT, &::mbg::launch_step<T, 2, LEV, C, NT>, 0, \
+        &::mbg::launch_persist<T, 2, LEV, C, NT>);
 #define MBG_REG_CVR_P(T, LEV, C, NT)                                           \
     static const bool MBG_CAT(mbg_reg_, __LINE__) = ::mbg::register_kernel<T>( \
         ::mbg::ALGO_CVR, LEV, C, NT, &::mbg::launch_step<T, 1, LEV, C, NT>, 0,  \
         &::mbg::launch_persist<T, 1, LEV, C, NT>);
-
-#define MBG_REG_CVR_TC(LEV)                                                       \
-    static const bool MBG_CAT(mbg_reg_, __LINE__) = ::mbg::register_kernel<float>( \
-        ::mbg::ALGO_CVR, LEV, 1, ::mbg::tc::M, &::mbg::launch_step_tc<LEV>);
 
 #define MBG_REG_CVR2_BULK(C, NT)                                                  \
     static const bool MBG_CAT(mbg_reg_, __LINE__) = ::mbg::register_kernel<float>( \

@@ -868,8 +868,11 @@ __device__ __forceinline__ void cayley_update(T (&rho)[N * N], T e, T& pout, con
 //   s = D(rh);  A(e) Y = W (LU without pivoting: A's Hermitian part is I);
 //   dU = 2 i e Y;  Z = dU s;  E = Z (U0 + dU)^H + U0 Z^H.
 // One renormalisation of the pairs per step; P = gP . rho.
+//
+// The field-dependent part, inc = D(E(D rh)):
 template<int N>
-__device__ __forceinline__ void cayley_update_df(float (&rh)[N * N], float (&rl)[N * N], float e, float& pout, const float* cf)
+__device__ __forceinline__ void cayley_increment_df(const float (&rh)[N * N], float e, const float* cf,
+                                                    float (&inc)[N * N])
 {
     typedef cpx_f cx;
     constexpr int NN = N * N;
@@ -1015,8 +1018,7 @@ __device__ __forceinline__ void cayley_update_df(float (&rh)[N * N], float (&rl)
                 ev[N + 2 * q + 1] = ei;
             }
         }
-    // increments: D(E) + B0 rh (high part), B0l rh (low part)
-    float inc[NN], incl[NN];
+    // D(E)
 #pragma unroll
     for (int i = 0; i < N; i++) {
         float v = ev[i];
@@ -1030,6 +1032,16 @@ __device__ __forceinline__ void cayley_update_df(float (&rh)[N * N], float (&rl)
         inc[N + 2 * q] = fmaf(dd, ev[N + 2 * q], ev[N + 2 * q]);
         inc[N + 2 * q + 1] = fmaf(dd, ev[N + 2 * q + 1], ev[N + 2 * q + 1]);
     }
+}
+
+template<int N>
+__device__ __forceinline__ void cayley_update_df(float (&rh)[N * N], float (&rl)[N * N], float e, float& pout, const float* cf)
+{
+    constexpr int NN = N * N;
+    const pre::cay_layout L = pre::make_cay_layout(N);
+    // increments: D(E) + B0 rh (high part), B0l rh (low part)
+    float inc[NN], incl[NN];
+    cayley_increment_df<N>(rh, e, cf, inc);
     if (cf[L.blockB0] != 0.0f) {
         // diagonal H0: B0 is block-diagonal (populations; each coherence's
         // 2 x 2 block), the same sums without their exact zero terms

@@ -1,5 +1,7 @@
-// Tensor-core form of the coherence-vector step for 4 to 6 levels
-// (FP32 kernels, uniform tiles, 128 points per CTA, one per thread).
+// Tensor-core form of the density steps for 4 to 6 levels (FP32 kernels,
+// uniform tiles, 128 points per CTA, one per thread): the coherence vector's
+// propagator product, and the field-free product of the Cayley step, of the
+// same form.
 //
 // Each step's correction Bd v + k (after the field rotation; see
 // cvr_layout) is, over the CTA's 128 points, the product
@@ -87,6 +89,7 @@ struct ctx {
     uint32_t mbar;
     uint32_t phase;
     uint32_t wait_limit;  // polls of a completion wait
+    volatile int* fail;   // shared: a completion wait of this CTA ran out
 };
 
 __device__ __forceinline__ void mma_tf32(uint32_t d, uint64_t a, uint64_t b, uint32_t id, uint32_t acc)
@@ -141,8 +144,7 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16])
     for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
 }
 
-// Stage the B operands from the material block in global memory (layout of
-// make_cvr_layout: Bd at FDTD_END, Bdl after it, both V x V row-major):
+// Stage the B operands from the material block in global memory:
 // Bd + Bdl = B_hi + B_lo + B_rest with B_hi and B_lo TF32 numbers (rounded
 // to nearest) and B_rest the FP32 remainder. The tensor cores read only a
 // TF32 number's bits, so a B_lo that was not itself a TF32 number would be
@@ -150,12 +152,11 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16])
 // Bdl correction. The second accumulator takes B_rest (D1 = A_hi B_rest).
 // Rows n >= V and columns k >= V are zero. Called by all threads; a barrier
 // must follow.
+// (bd, bdl: V x V, rows ld apart.)
 template<int V>
-__device__ __forceinline__ void stage_b(const ctx& c, const float* mat)
+__device__ __forceinline__ void stage_b(const ctx& c, const float* bd, const float* bdl, int ld)
 {
     using S = shape<V>;
-    const float* bd = mat + pre::FDTD_END;
-    const float* bdl = bd + V * V;
     for (int e = threadIdx.x; e < S::N * S::KC; e += M) {
         const int n = e / S::KC, kc = e % S::KC;
         float h[4], l[4], dl[4];
@@ -163,11 +164,11 @@ __device__ __forceinline__ void stage_b(const ctx& c, const float* mat)
         for (int q = 0; q < 4; q++) {
             const int k = kc * 4 + q;
             const bool in = n < V && k < V;
-            const float b = in ? bd[n * V + k] : 0.0f;
+            const float b = in ? bd[n * ld + k] : 0.0f;
             h[q] = tf32_hi(b);
             const float r = b - h[q];           // exact
             l[q] = tf32_hi(r);
-            dl[q] = (r - l[q]) + (in ? bdl[n * V + k] : 0.0f);
+            dl[q] = (r - l[q]) + (in ? bdl[n * ld + k] : 0.0f);
         }
         const uint32_t o = chunk<V>(n, kc);
         st16(c.b_hi + o, h[0], h[1], h[2], h[3]);
@@ -203,11 +204,13 @@ __device__ __forceinline__ void write_row(const ctx& c, const float (&x)[V])
     });
 }
 
-// D0 = A_hi Bhi^T + A_hi Blo^T + A_lo Bhi^T, D1 = A_hi Bdl^T; returns false
-// when the completion wait ran out. Called by all threads of the CTA after
-// write_row.
+// D0 = A_hi Bhi^T + A_hi Blo^T + A_lo Bhi^T, D1 = A_hi Bdl^T: issued by
+// product_issue (all threads of the CTA, after write_row), complete after
+// product_wait. A wait that runs out is noted in *fail and the CTA goes on
+// without waiting again (its results are void; every thread keeps meeting
+// the same barriers).
 template<int V>
-__device__ __forceinline__ bool product(ctx& c)
+__device__ __forceinline__ void product_issue(const ctx& c)
 {
     using S = shape<V>;
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -227,12 +230,13 @@ __device__ __forceinline__ bool product(ctx& c)
         asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(c.mbar)
                      : "memory");
     }
-    const bool ok = mbar_wait(c.mbar, c.phase, c.wait_limit);
+}
+
+__device__ __forceinline__ void product_wait(ctx& c)
+{
+    if (*c.fail == 0 && !mbar_wait(c.mbar, c.phase, c.wait_limit)) *c.fail = 1;
     c.phase ^= 1u;
     fence_after();
-    // the same answer in every thread, so that a time-out ends the tile in
-    // all of them
-    return __syncthreads_and(ok) != 0;
 }
 
 // Row threadIdx.x of D0 and D1, 16 columns at a time: f(i, D0[i], D1[i])
@@ -295,12 +299,13 @@ __device__ __forceinline__ void rotate_df(float (&uh)[V], float (&ul)[V], float 
 // the CTA call it (threads without a point pass zeros and discard the
 // result).
 template<int V, class CF>
-__device__ __forceinline__ bool cvr_update_df_tc(
+__device__ __forceinline__ void cvr_update_df_tc(
     ctx& c, float (&uh)[V], float (&ul)[V], float e, float& pout, const CF& cf)
 {
     rotate_df<V>(uh, ul, e, cf);
     write_row<V>(c, uh);
-    if (!product<V>(c)) return false;
+    product_issue<V>(c);
+    product_wait(c);
     float pp = cf.p0();
     consume_row<V>(c, [&](auto I, float d, float dl) {
         constexpr int i = decltype(I)::value;
@@ -310,7 +315,35 @@ __device__ __forceinline__ bool cvr_update_df_tc(
     });
     pout = pp;
     fence_before();   // the reads of D above precede the next product's MMAs
-    return true;
+}
+
+// The FP32 Cayley step of cayley_update_df with the field-free product B0 rho
+// (the N^2 x N^2 matrix and its low words: 2 N^4 of the step's FMAs, each
+// with a coefficient from shared memory) on the tensor cores. The product
+// needs only the state before the step, so its MMAs run while the CUDA cores
+// solve for the field-dependent part. One 6-level run of 65,536 points: 34.4
+// -> 21.5 us a step, what is left being the solve and its products on 8
+// warps per SM (255 registers).
+template<int N>
+__device__ __forceinline__ void cayley_update_df_tc(
+    ctx& c, float (&rh)[N * N], float (&rl)[N * N], float e, float& pout, const float* cf)
+{
+    constexpr int NN = N * N;
+    const pre::cay_layout L = pre::make_cay_layout(N);
+    write_row<NN>(c, rh);
+    product_issue<NN>(c);
+    float inc[NN];
+    cayley_increment_df<N>(rh, e, cf, inc);
+    product_wait(c);
+    float acc = 0.0f;
+    consume_row<NN>(c, [&](auto I, float d, float dl) {
+        constexpr int i = decltype(I)::value;
+        df_acc(rh[i], rl[i], inc[i] + d, dl);
+        df_renorm(rh[i], rl[i]);
+        acc = fmaf(cf[L.gP + i], rh[i], fmaf(cf[L.gP + i], rl[i], acc));
+    });
+    pout = acc;
+    fence_before();   // as above
 }
 
 // The same step on the CUDA cores with the point's own coefficients

@@ -284,9 +284,8 @@ __device__ __forceinline__ void for_records(const kparams<T>& p, const run_desc&
 
 namespace mbg {
 
-// Returns false when a tensor-core wait ran out (TC kernels only).
 template<typename T, int ALGO, int LEV, int C, int NT, bool UNIFORM, bool TC = false>
-__device__ __forceinline__ bool tile_steps(
+__device__ __forceinline__ void tile_steps(
     const kparams<T>& p,
     const tile_desc& td,
     const run_desc& rd,
@@ -322,7 +321,7 @@ __device__ __forceinline__ bool tile_steps(
     constexpr int D = density_len<ALGO, LEV>::value;
     constexpr int NW = NT / 32;
     constexpr bool TCU = TC && UNIFORM;  // density products on the tensor cores
-    static_assert(!TC || (DF && ALGO == 1 && D >= 15 && C == 1 && NT == tc::M), "TC kernel shape");
+    static_assert(!TC || (DF && ALGO != 0 && D >= 15 && C == 1 && NT == tc::M), "TC kernel shape");
     // 2-level coefficients live in registers on uniform tiles; for 4 and more
     // levels uniform tiles hold the padded copy of cvr_pad in shared memory
     constexpr bool REGCOEF = UNIFORM && ALGO == 1 && D == 3;
@@ -484,8 +483,12 @@ __device__ __forceinline__ bool tile_steps(
                 const bool act = M[0] >= 0;
                 const float e = act ? E[0] + El[0] : 0.0f;
                 float pn = 0.0f;
-                const tc::coef_small<D> cf{ sh_coef };
-                if (!tc::cvr_update_df_tc<D>(*tcc, R[0], Rl[0], e, pn, cf)) return false;
+                if constexpr (ALGO == 1) {
+                    const tc::coef_small<D> cf{ sh_coef };
+                    tc::cvr_update_df_tc<D>(*tcc, R[0], Rl[0], e, pn, cf);
+                } else {
+                    tc::cayley_update_df_tc<LEV>(*tcc, R[0], Rl[0], e, pn, sh_coef);
+                }
                 if (act) {
                     P[0] = pn;
                 } else {
@@ -607,7 +610,15 @@ __device__ __forceinline__ bool tile_steps(
                 if constexpr (DF) Hl[j] = T(0);
             }
     }
-    return true;
+}
+
+// Leading entries of the material block (ALGO 1: of coef_small) that a
+// tensor-core kernel's uniform tile stages in shared memory; the operands
+// follow at the next multiple of 128 bytes
+template<int ALGO, int LEV>
+MBG_HD int tc_coef_len()
+{
+    return ALGO == 1 ? tc::coef_small<density_len<ALGO, LEV>::value>::len : pre::make_cay_layout(LEV).B0;
 }
 
 // Tensor memory columns, completion barrier and its phase of a CTA of the
@@ -615,9 +626,10 @@ __device__ __forceinline__ bool tile_steps(
 struct tc_res {
     uint32_t tmem, mbar;
     uint32_t* phase;  // shared: the barrier's phase between tiles
+    int* fail;        // shared: a completion wait ran out
 };
 
-__device__ __forceinline__ tc_res tc_acquire(uint32_t* tmem_sh, uint64_t* mbar, uint32_t* phase_sh)
+__device__ __forceinline__ tc_res tc_acquire(uint32_t* tmem_sh, uint64_t* mbar, uint32_t* phase_sh, int* fail_sh)
 {
     if (threadIdx.x < 32) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
@@ -631,11 +643,12 @@ __device__ __forceinline__ tc_res tc_acquire(uint32_t* tmem_sh, uint64_t* mbar, 
                      : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         *phase_sh = 0;
+        *fail_sh = 0;
     }
     tc::fence_before();
     __syncthreads();
     tc::fence_after();
-    return tc_res{ *tmem_sh, (uint32_t) __cvta_generic_to_shared(mbar), phase_sh };
+    return tc_res{ *tmem_sh, (uint32_t) __cvta_generic_to_shared(mbar), phase_sh, fail_sh };
 }
 
 __device__ __forceinline__ void tc_release(const tc_res& r)
@@ -771,9 +784,11 @@ __device__ __forceinline__ void step_body(const kparams<T>& p, uint32_t tile, ui
     const bool uniform = td.uniform_mat >= 0;
     if (uniform) {
         const T* src = p.mc + (uint64_t) td.uniform_mat * p.mstride;
-        if constexpr (TC) {
+        if constexpr (TC && ALGO == 1) {
             using Ls = tc::coef_small<D>;
             for (int i = threadIdx.x; i < Ls::len; i += NT) sh_coef[i] = src[Ls::source(i)];
+        } else if constexpr (TC) {
+            for (int i = threadIdx.x; i < tc_coef_len<ALGO, LEV>(); i += NT) sh_coef[i] = src[i];
         } else if constexpr (ALGO == 1 && D >= 15) {
             using Lp = cvr_pad<T, D>;
             for (int i = threadIdx.x; i < Lp::len; i += NT) {
@@ -795,7 +810,7 @@ __device__ __forceinline__ void step_body(const kparams<T>& p, uint32_t tile, ui
     if constexpr (TC) {
         tc::fence_after();
         const uint32_t sbase = (uint32_t) __cvta_generic_to_shared(smem_raw);
-        const uint32_t ops = (sbase + (uint32_t) (tc::coef_small<D>::len * sizeof(T)) + 127u) & ~127u;
+        const uint32_t ops = (sbase + (uint32_t) (tc_coef_len<ALGO, LEV>() * sizeof(T)) + 127u) & ~127u;
         tcc.rows = reinterpret_cast<float*>(smem_raw + (ops - sbase));
         using TS = tc::shape<D>;
         tcc.a_hi = ops;
@@ -807,7 +822,16 @@ __device__ __forceinline__ void step_body(const kparams<T>& p, uint32_t tile, ui
         tcc.mbar = res.mbar;
         tcc.phase = *res.phase;
         tcc.wait_limit = p.wait_limit ? p.wait_limit : tc::WAIT_LIMIT;
-        if (uniform) tc::stage_b<D>(tcc, p.mc + (uint64_t) td.uniform_mat * p.mstride);
+        tcc.fail = res.fail;
+        if (uniform) {
+            const T* mat = p.mc + (uint64_t) td.uniform_mat * p.mstride;
+            if constexpr (ALGO == 1) {
+                tc::stage_b<D>(tcc, mat + pre::FDTD_END, mat + pre::FDTD_END + D * D, D);
+            } else {
+                const pre::cay_layout L = pre::make_cay_layout(LEV);
+                tc::stage_b<D>(tcc, mat + L.B0, mat + L.B0l, L.NP);
+            }
+        }
     }
 
     if (uniform) {
@@ -826,10 +850,8 @@ __device__ __forceinline__ void step_body(const kparams<T>& p, uint32_t tile, ui
             else
                 run(std::false_type{}, std::true_type{});
         } else {
-            const bool ok = tile_steps<T, ALGO, LEV, C, NT, true, TC>(p, td, rd, l0, nsteps, step0, E, El, H, Hl,
-                                                                      P, R, Rl, M, sh_coef, tl, sv, own, sh_a,
-                                                                      sh_al, sh_b, sh_bl, &tcc);
-            if (!ok && threadIdx.x == 0) atomicOr(p.status, STATUS_TC_WAIT);
+            tile_steps<T, ALGO, LEV, C, NT, true, TC>(p, td, rd, l0, nsteps, step0, E, El, H, Hl, P, R, Rl, M, sh_coef,
+                                                      tl, sv, own, sh_a, sh_al, sh_b, sh_bl, &tcc);
         }
     } else {
         tile_steps<T, ALGO, LEV, C, NT, false>(p, td, rd, l0, nsteps, step0, E, El, H, Hl, P, R, Rl, M,
@@ -840,6 +862,7 @@ __device__ __forceinline__ void step_body(const kparams<T>& p, uint32_t tile, ui
         // CTA continues from it (the barrier before its first product
         // orders this write)
         if (threadIdx.x == 0) *res.phase = tcc.phase;
+        if (*tcc.fail) atomicOr(p.status, STATUS_TC_WAIT);
     }
 
     // Cayley, FP32: renormalise the trace to that of the initial density
@@ -921,20 +944,25 @@ __device__ __forceinline__ void step_body(const kparams<T>& p, uint32_t tile, ui
 // The time-step kernels. The CUDA-core kernels leave the register budget to
 // the compiler (a minimum-blocks hint would raise the 2-level kernels to
 // more registers and one CTA per SM); the tensor-core kernels ask for 3
-// CTAs per SM (4 for 4 levels), which needs the in-place update's budget.
+// CTAs per SM (4 for 4 levels), which needs the in-place update's budget,
+// the Cayley ones, whose solve needs the registers, for 2 (3 for 4 levels).
 template<typename T, int ALGO, int LEV, int C, int NT>
 __global__ void __launch_bounds__(NT) step_kernel(const kparams<T> p)
 {
     step_body<T, ALGO, LEV, C, NT, false>(p, blockIdx.x, p.launch_idx, false, tc_res{});
 }
 
-template<int LEV>
-__global__ void __launch_bounds__(tc::M, LEV <= 4 ? 4 : 3) step_kernel_tc(const kparams<float> p)
+// CTAs per SM of the tensor-core kernels
+constexpr int tc_blocks(int algo, int lev) { return algo == 2 ? (lev <= 4 ? 3 : 2) : lev <= 4 ? 4 : 3; }
+
+template<int ALGO, int LEV>
+__global__ void __launch_bounds__(tc::M, tc_blocks(ALGO, LEV)) step_kernel_tc(const kparams<float> p)
 {
     __shared__ __align__(8) uint64_t mbar;
     __shared__ uint32_t tmem_sh, phase_sh;
-    const tc_res r = tc_acquire(&tmem_sh, &mbar, &phase_sh);
-    step_body<float, 1, LEV, 1, tc::M, true>(p, blockIdx.x, p.launch_idx, false, r);
+    __shared__ int fail_sh;
+    const tc_res r = tc_acquire(&tmem_sh, &mbar, &phase_sh, &fail_sh);
+    step_body<float, ALGO, LEV, 1, tc::M, true>(p, blockIdx.x, p.launch_idx, false, r);
     tc_release(r);
 }
 
@@ -1029,14 +1057,15 @@ __global__ void __launch_bounds__(NT) step_kernel_persist(const kparams<T> p, co
     persist_loop<T, ALGO, LEV, C, NT, false>(p, q, tc_res{});
 }
 
-template<int LEV>
-__global__ void __launch_bounds__(tc::M, LEV <= 4 ? 4 : 3)
+template<int ALGO, int LEV>
+__global__ void __launch_bounds__(tc::M, tc_blocks(ALGO, LEV))
     step_kernel_persist_tc(const kparams<float> p, const persist_params q)
 {
     __shared__ __align__(8) uint64_t mbar;
     __shared__ uint32_t tmem_sh, phase_sh;
-    const tc_res r = tc_acquire(&tmem_sh, &mbar, &phase_sh);
-    persist_loop<float, 1, LEV, 1, tc::M, true>(p, q, r);
+    __shared__ int fail_sh;
+    const tc_res r = tc_acquire(&tmem_sh, &mbar, &phase_sh, &fail_sh);
+    persist_loop<float, ALGO, LEV, 1, tc::M, true>(p, q, r);
     tc_release(r);
 }
 
