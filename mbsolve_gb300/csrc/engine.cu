@@ -625,6 +625,9 @@ public:
             cudaEventDestroy(e.a);
             cudaEventDestroy(e.b);
         }
+        for (auto& e : pin_done_)
+            if (e) cudaEventDestroy(e);
+        if (pin_) cudaFreeHost(pin_);
         if (stream_) cudaStreamDestroy(stream_);
     }
 
@@ -832,19 +835,51 @@ public:
         const run_setup& rs = runs_.at(run);
         if (k >= rs.records.size()) throw invalid_argument("result index out of range");
         const auto& rc = rs.records[k];
-        uint64_t size = (uint64_t) rc.d.cols * rc.d.rows;
-        std::vector<T> tmp(size);
+        const uint64_t size = (uint64_t) rc.d.cols * rc.d.rows;
+        const T* src = scratch_.p + scratch_base_[run] + rc.d.offset;
         MBG_CK(cudaStreamSynchronize(stream_));
-        MBG_CK(cudaMemcpy(tmp.data(), scratch_.p + scratch_base_[run] + rc.d.offset,
-                          size * sizeof(T), cudaMemcpyDeviceToHost));
-        for (uint64_t i = 0; i < size; i++) re[i] = (double) tmp[i];
+        copy_values(src, size, re);
         if (im) {
-            if (rc.is_complex) {
-                MBG_CK(cudaMemcpy(tmp.data(), scratch_.p + scratch_base_[run] + rc.d.offset + size,
-                                  size * sizeof(T), cudaMemcpyDeviceToHost));
-                for (uint64_t i = 0; i < size; i++) im[i] = (double) tmp[i];
-            } else {
+            if (rc.is_complex)
+                copy_values(src + size, size, im);
+            else
                 std::fill(im, im + size, 0.0);
+        }
+    }
+
+    // n device values to doubles on the host; the stream is idle. Large FP32
+    // records come through two pinned chunks, one converted while the other
+    // arrives: a pageable copy of the whole record into a vector wrote and
+    // read it once more through fresh pages (3-level Lambda run with two
+    // records of 2 x 1,048,576 values, 200 steps: 13.4 -> 12.1 ms).
+    void copy_values(const T* src, uint64_t n, double* out)
+    {
+        if constexpr (sizeof(T) == sizeof(double)) {
+            MBG_CK(cudaMemcpy(out, src, n * sizeof(T), cudaMemcpyDeviceToHost));
+        } else {
+            if (n <= PIN_MIN) {
+                std::vector<T> tmp(n);
+                MBG_CK(cudaMemcpy(tmp.data(), src, n * sizeof(T), cudaMemcpyDeviceToHost));
+                for (uint64_t i = 0; i < n; i++) out[i] = (double) tmp[i];
+                return;
+            }
+            if (!pin_) MBG_CK(cudaMallocHost((void**) &pin_, 2 * PIN_CHUNK * sizeof(T)));
+            for (auto& e : pin_done_)
+                if (!e) MBG_CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+            const uint64_t chunks = (n + PIN_CHUNK - 1) / PIN_CHUNK;
+            auto count = [&](uint64_t k) { return std::min<uint64_t>(PIN_CHUNK, n - k * PIN_CHUNK); };
+            auto fetch = [&](uint64_t k) {
+                MBG_CK(cudaMemcpyAsync(pin_ + (k & 1) * PIN_CHUNK, src + k * PIN_CHUNK, count(k) * sizeof(T),
+                                       cudaMemcpyDeviceToHost, stream_));
+                MBG_CK(cudaEventRecord(pin_done_[k & 1], stream_));
+            };
+            fetch(0);
+            for (uint64_t k = 0; k < chunks; k++) {
+                if (k + 1 < chunks) fetch(k + 1);
+                MBG_CK(cudaEventSynchronize(pin_done_[k & 1]));
+                const T* t = pin_ + (k & 1) * PIN_CHUNK;
+                double* o = out + k * PIN_CHUNK;
+                for (uint64_t i = 0, m = count(k); i < m; i++) o[i] = (double) t[i];
             }
         }
     }
@@ -925,6 +960,10 @@ private:
     uint64_t launches_ = 0;  // every kernel launched by advance()/copies
 
     cudaEvent_t region_[2] = { nullptr, nullptr };
+    // copy_values: two pinned chunks, from the first large record on
+    static constexpr uint64_t PIN_MIN = 1u << 15, PIN_CHUNK = 1u << 18;
+    T* pin_ = nullptr;
+    cudaEvent_t pin_done_[2] = { nullptr, nullptr };
 
 public:
     uint64_t launches() const override { return launches_; }

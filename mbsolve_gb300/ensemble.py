@@ -78,11 +78,11 @@ class ensemble:
             r, c, z = C.c_uint32(), C.c_uint32(), C.c_int32()
             _native.check(self._L.mbg_ensemble_result_shape(
                 self._h, run, k, C.byref(r), C.byref(c), C.byref(z)))
-            re = np.zeros(r.value * c.value)
-            im = np.zeros(r.value * c.value)
+            re = np.empty(r.value * c.value)
+            im = np.zeros(r.value * c.value)  # untouched unless complex
             _native.check(self._L.mbg_ensemble_copy_result(
                 self._h, run, k, re.ctypes.data_as(T.PD),
-                im.ctypes.data_as(T.PD)))
+                im.ctypes.data_as(T.PD) if z.value else None))
             out.append(mb.result(rec.get_name(), c.value, r.value,
                                  bool(z.value), re, im))
         return out

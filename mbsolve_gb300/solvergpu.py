@@ -53,10 +53,11 @@ class solver_gpu_fdtd(mb.solver):
             # keep the error text: the copies below overwrite it
             err = _native.MbgError(rc, self._L.mbg_last_error().decode())
         for k, res in enumerate(self._results):
-            re = np.zeros(res.get_count())
-            im = np.zeros(res.get_count())
+            re = np.empty(res.get_count())
+            im = np.zeros(res.get_count())  # untouched unless complex
             crc = self._L.mbg_solver_copy_result(
-                self._h, k, re.ctypes.data_as(T.PD), im.ctypes.data_as(T.PD))
+                self._h, k, re.ctypes.data_as(T.PD),
+                im.ctypes.data_as(T.PD) if res.is_complex() else None)
             if crc != T.MBG_OK:
                 if rc == T.MBG_OK:
                     _native.check(crc)
