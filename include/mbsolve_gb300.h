@@ -269,7 +269,8 @@ int mbg_solver_grid(const mbg_solver* s, mbg_grid* out);
  * of the persistent kernel, 2^22 for a tensor-core or bulk-copy
  * completion). MBG_TEST_STALL_PERSIST=1 exists for tests only: every wait
  * of the persistent kernel then asks for progress no tile reaches and runs
- * out. */
+ * out; likewise MBG_TEST_STALL_TC=1, with which every tensor-core completion
+ * wait gives up without polling. */
 int mbg_solver_run(mbg_solver* s);
 
 /* Results, one per scenario record in record order (solver_cpu_fdtd.tpp:

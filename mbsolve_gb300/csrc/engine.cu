@@ -611,6 +611,7 @@ public:
         // bound of the kernels' device-side waits (polls), and the test
         // switch that makes every persistent-kernel wait run out
         if (const char* w = std::getenv("MBG_WAIT_LIMIT")) wait_limit_ = (uint32_t) std::strtoul(w, nullptr, 10);
+        if (const char* w = std::getenv("MBG_TEST_STALL_TC")) tc_stall_ = (w[0] == '1') ? 1u : 0u;
         if (const char* w = std::getenv("MBG_TEST_STALL_PERSIST")) stall_ = (w[0] == '1') ? (1u << 30) : 0u;
         MBG_CK(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
         setup();
@@ -943,6 +944,7 @@ private:
     uint64_t digest_ = 0;  // describe_digest(runs_), for checkpoints
     uint32_t wait_limit_ = 0;  // MBG_WAIT_LIMIT (0: the kernels' defaults)
     uint32_t stall_ = 0;       // MBG_TEST_STALL_PERSIST
+    uint32_t tc_stall_ = 0;    // MBG_TEST_STALL_TC
     persist_fn<T> pfn_ = nullptr;
     int persist_ = 0;
     dbuf<unsigned long long> step_, step_zero_;
@@ -1363,6 +1365,7 @@ private:
         p.record = record ? 1 : 0;
         p.status = status_.p;
         p.wait_limit = wait_limit_;
+        p.tc_stall = tc_stall_;
         return p;
     }
 

@@ -76,6 +76,7 @@ struct kparams {
     int record;           // 0 while autotuning
     uint32_t* status;
     uint32_t wait_limit;  // polls of a bounded device wait (0: the kernel's default)
+    uint32_t tc_stall;    // tests only: tensor-core completion waits give up without polling
 };
 
 // ------------------------------------------------------------ helpers

@@ -20,7 +20,9 @@
 // K-adjacent core matrices, K/4 x 128 bytes between 8-row groups).
 //
 // One thread issues the MMAs and commits them to an mbarrier; every wait is
-// bounded and a time-out stops the tile (status flag) instead of hanging.
+// bounded. After a time-out (status flag) the CTA issues no further product:
+// at most one is outstanding, and it is waited for once more, bounded again,
+// before the TMEM is given back.
 #pragma once
 
 #include <cstdint>
@@ -121,6 +123,12 @@ __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity, uint32
     return false;
 }
 
+// arrives on mbar when every MMA this thread has issued is complete
+__device__ __forceinline__ void commit(uint32_t mbar)
+{
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
+}
+
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
@@ -206,9 +214,9 @@ __device__ __forceinline__ void write_row(const ctx& c, const float (&x)[V])
 
 // D0 = A_hi Bhi^T + A_hi Blo^T + A_lo Bhi^T, D1 = A_hi Bdl^T: issued by
 // product_issue (all threads of the CTA, after write_row), complete after
-// product_wait. A wait that runs out is noted in *fail and the CTA goes on
-// without waiting again (its results are void; every thread keeps meeting
-// the same barriers).
+// product_wait. A wait that runs out is noted in *fail; the CTA then goes
+// through its remaining steps without products or waits (its results are
+// void; every thread keeps meeting the same barriers).
 template<int V>
 __device__ __forceinline__ void product_issue(const ctx& c)
 {
@@ -216,7 +224,8 @@ __device__ __forceinline__ void product_issue(const ctx& c)
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     fence_before();
     __syncthreads();
-    if (threadIdx.x == 0) {
+    // (*fail is set in product_wait, before this barrier)
+    if (threadIdx.x == 0 && *c.fail == 0) {
         fence_after();
         constexpr uint32_t id = idesc<V>();
 #pragma unroll
@@ -227,8 +236,7 @@ __device__ __forceinline__ void product_issue(const ctx& c)
             mma_tf32(c.tmem, desc<V>(c.a_lo + o), desc<V>(c.b_hi + o), id, 1u);
             mma_tf32(c.tmem + D1_COL, desc<V>(c.a_hi + o), desc<V>(c.b_dl + o), id, ks > 0 ? 1u : 0u);
         }
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(c.mbar)
-                     : "memory");
+        commit(c.mbar);
     }
 }
 

@@ -622,7 +622,8 @@ MBG_HD int tc_coef_len()
 }
 
 // Tensor memory columns, completion barrier and its phase of a CTA of the
-// tensor-core kernels (allocated once per CTA by the kernel wrappers).
+// tensor-core kernels (allocated once per CTA by the kernel wrappers; the
+// second barrier, 8 bytes on, is tc_release's).
 struct tc_res {
     uint32_t tmem, mbar;
     uint32_t* phase;  // shared: the barrier's phase between tiles
@@ -639,8 +640,9 @@ __device__ __forceinline__ tc_res tc_acquire(uint32_t* tmem_sh, uint64_t* mbar, 
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     if (threadIdx.x == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((uint32_t) __cvta_generic_to_shared(mbar))
-                     : "memory");
+        for (int i = 0; i < 2; i++)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((uint32_t) __cvta_generic_to_shared(mbar + i))
+                         : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         *phase_sh = 0;
         *fail_sh = 0;
@@ -656,6 +658,13 @@ __device__ __forceinline__ void tc_release(const tc_res& r)
     tc::fence_before();
     __syncthreads();
     if (threadIdx.x < 32) {
+        // after a time-out a product may still be reading shared memory and
+        // writing TMEM: the thread that issued it waits for it
+        if (threadIdx.x == 0 && *r.fail) {
+            tc::commit(r.mbar + 8u);
+            tc::mbar_wait(r.mbar + 8u, 0u, tc::WAIT_LIMIT);
+        }
+        __syncwarp();
         tc::fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(r.tmem), "r"(tc::TMEM_COLS)
                      : "memory");
@@ -821,9 +830,9 @@ __device__ __forceinline__ void step_body(const kparams<T>& p, uint32_t tile, ui
         tcc.tmem = res.tmem;
         tcc.mbar = res.mbar;
         tcc.phase = *res.phase;
-        tcc.wait_limit = p.wait_limit ? p.wait_limit : tc::WAIT_LIMIT;
+        tcc.wait_limit = p.tc_stall ? 0u : p.wait_limit ? p.wait_limit : tc::WAIT_LIMIT;
         tcc.fail = res.fail;
-        if (uniform) {
+        if (uniform && *tcc.fail == 0) {
             const T* mat = p.mc + (uint64_t) td.uniform_mat * p.mstride;
             if constexpr (ALGO == 1) {
                 tc::stage_b<D>(tcc, mat + pre::FDTD_END, mat + pre::FDTD_END + D * D, D);
@@ -958,10 +967,10 @@ constexpr int tc_blocks(int algo, int lev) { return algo == 2 ? (lev <= 4 ? 3 : 
 template<int ALGO, int LEV>
 __global__ void __launch_bounds__(tc::M, tc_blocks(ALGO, LEV)) step_kernel_tc(const kparams<float> p)
 {
-    __shared__ __align__(8) uint64_t mbar;
+    __shared__ __align__(8) uint64_t mbar[2];
     __shared__ uint32_t tmem_sh, phase_sh;
     __shared__ int fail_sh;
-    const tc_res r = tc_acquire(&tmem_sh, &mbar, &phase_sh, &fail_sh);
+    const tc_res r = tc_acquire(&tmem_sh, mbar, &phase_sh, &fail_sh);
     step_body<float, ALGO, LEV, 1, tc::M, true>(p, blockIdx.x, p.launch_idx, false, r);
     tc_release(r);
 }
@@ -1061,10 +1070,10 @@ template<int ALGO, int LEV>
 __global__ void __launch_bounds__(tc::M, tc_blocks(ALGO, LEV))
     step_kernel_persist_tc(const kparams<float> p, const persist_params q)
 {
-    __shared__ __align__(8) uint64_t mbar;
+    __shared__ __align__(8) uint64_t mbar[2];
     __shared__ uint32_t tmem_sh, phase_sh;
     __shared__ int fail_sh;
-    const tc_res r = tc_acquire(&tmem_sh, &mbar, &phase_sh, &fail_sh);
+    const tc_res r = tc_acquire(&tmem_sh, mbar, &phase_sh, &fail_sh);
     persist_loop<float, ALGO, LEV, 1, tc::M, true>(p, q, r);
     tc_release(r);
 }
