@@ -240,11 +240,18 @@ __device__ __forceinline__ void product_issue(const ctx& c)
     }
 }
 
-__device__ __forceinline__ void product_wait(ctx& c)
+// The vote makes the warp whole again after the polling loop, whose lanes
+// leave it one by one: the TMEM loads that follow are warp-wide
+// (.sync.aligned). False, for the whole warp, where the product is not known
+// to be complete: its accumulators are not to be read.
+__device__ __forceinline__ bool product_wait(ctx& c)
 {
-    if (*c.fail == 0 && !mbar_wait(c.mbar, c.phase, c.wait_limit)) *c.fail = 1;
+    const bool ok = *c.fail == 0 && mbar_wait(c.mbar, c.phase, c.wait_limit);
+    if (!ok) *c.fail = 1;
     c.phase ^= 1u;
+    const bool all = __all_sync(0xffffffffu, ok);
     fence_after();
+    return all;
 }
 
 // Row threadIdx.x of D0 and D1, 16 columns at a time: f(i, D0[i], D1[i])
@@ -305,7 +312,7 @@ __device__ __forceinline__ void rotate_df(float (&uh)[V], float (&ul)[V], float 
 // on the tensor cores. The product reads its own copy of the vector
 // (shared memory), so the registers are updated in place. All threads of
 // the CTA call it (threads without a point pass zeros and discard the
-// result).
+// result). pout stays as it was when the product did not complete.
 template<int V, class CF>
 __device__ __forceinline__ void cvr_update_df_tc(
     ctx& c, float (&uh)[V], float (&ul)[V], float e, float& pout, const CF& cf)
@@ -313,7 +320,7 @@ __device__ __forceinline__ void cvr_update_df_tc(
     rotate_df<V>(uh, ul, e, cf);
     write_row<V>(c, uh);
     product_issue<V>(c);
-    product_wait(c);
+    if (!product_wait(c)) return;
     float pp = cf.p0();
     consume_row<V>(c, [&](auto I, float d, float dl) {
         constexpr int i = decltype(I)::value;
@@ -342,7 +349,7 @@ __device__ __forceinline__ void cayley_update_df_tc(
     product_issue<NN>(c);
     float inc[NN];
     cayley_increment_df<N>(rh, e, cf, inc);
-    product_wait(c);
+    if (!product_wait(c)) return;
     float acc = 0.0f;
     consume_row<NN>(c, [&](auto I, float d, float dl) {
         constexpr int i = decltype(I)::value;
