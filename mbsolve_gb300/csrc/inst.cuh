@@ -37,7 +37,7 @@ template<int ALGO, int LEV>
 size_t tc_smem()
 {
     return ((tc_coef_len<ALGO, LEV>() * sizeof(float) + 127) & ~(size_t) 127) + 128 +
-        tc::shape<density_len<ALGO, LEV>::value>::BYTES;
+        tc::shape<density_len<ALGO, LEV>::value, ALGO == 2>::BYTES;
 }
 
 template<int ALGO, int LEV>

@@ -208,6 +208,7 @@ struct cay_layout {
     int stage64;  // leading part the FP64 kernels use and stage
     int U0, Wk, NP, B0, B0l;
     int blockB0;  // 1: H0 is diagonal and B0 block-diagonal (see cay_free_step)
+    int maxB0;    // largest |entry| of B0 (the tensor-core form's grid)
     int stride;
 };
 
@@ -255,6 +256,8 @@ MBG_HD cay_layout make_cay_layout(int N)
     L.B0l = o;
     o += N * N * L.NP;
     L.blockB0 = o;
+    o += 1;
+    L.maxB0 = o;
     o += 1;
     L.stride = (o + 3) & ~3;
     return L;
@@ -1335,6 +1338,21 @@ MBG_HD void cay_free_step(const cay_layout& L, double* ws, double* out, const G&
             out[L.B0 + i * L.NP + v] = b;
             out[L.B0l + i * L.NP + v] = b - (double) (float) b;
         }
+    }
+    g.sync();
+    for (int i = g.rank; i < NN; i += g.size) {
+        double m = 0.0;
+        for (int v = 0; v < NN; v++) {
+            const double b = fabs(out[L.B0 + i * L.NP + v]);
+            m = b > m ? b : m;
+        }
+        r[i] = m;
+    }
+    g.sync();
+    if (g.rank == 0) {
+        double m = 0.0;
+        for (int i = 0; i < NN; i++) m = r[i] > m ? r[i] : m;
+        out[L.maxB0] = m;
     }
 }
 

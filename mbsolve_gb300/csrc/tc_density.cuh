@@ -1,7 +1,7 @@
 // Tensor-core form of the density steps for 4 to 6 levels (FP32 kernels,
 // uniform tiles, 128 points per CTA, one per thread): the coherence vector's
 // propagator product, and the field-free product of the Cayley step, of the
-// same form.
+// same form but in more words (write_row_fix).
 //
 // Each step's correction Bd v + k (after the field rotation; see
 // cvr_layout) is, over the CTA's 128 points, the product
@@ -34,10 +34,10 @@ namespace tc {
 
 constexpr int M = 128;                     // points per CTA (TMEM lanes)
 constexpr uint32_t WAIT_LIMIT = 1u << 22;
-constexpr uint32_t TMEM_COLS = 128;        // D0 at column 0, D1 at column 64
-constexpr uint32_t D1_COL = 64;
+constexpr uint32_t D1_COL = 64;            // D0 at column 0
 
-template<int V>
+// FIX: operands with a word on a common grid (write_row_fix)
+template<int V, bool FIX = false>
 struct shape {
     static constexpr int K = (V + 7) / 8 * 8;      // TF32: 8 per MMA
     static constexpr int N = (V + 15) / 16 * 16;   // M = 128 needs N % 16 == 0
@@ -45,9 +45,11 @@ struct shape {
     static constexpr uint32_t SBO = (uint32_t) KC * 128u;
     static constexpr uint32_t A_BYTES = (uint32_t) M * K * 4u;
     static constexpr uint32_t B_BYTES = (uint32_t) N * K * 4u;
-    // A_hi, A_lo, B_hi, B_lo, B_dl
-    static constexpr uint32_t BYTES = 2u * A_BYTES + 3u * B_BYTES;
+    // A_hi, A_lo, (FIX: A_fix, B_fix), B_hi, B_lo, B_dl
+    static constexpr uint32_t BYTES = (FIX ? 3u : 2u) * A_BYTES + (FIX ? 4u : 3u) * B_BYTES;
     static_assert(N <= 64, "two accumulators of N columns must fit 128 TMEM columns");
+    // FIX: four accumulators side by side (a power of two of columns)
+    static constexpr uint32_t TMEM_COLS = !FIX ? 2u * D1_COL : 4 * N > 128 ? 256u : 4 * N > 64 ? 128u : 64u;
 };
 
 // byte offset of the 16-byte chunk (row, kc) in a K-major operand
@@ -71,9 +73,9 @@ __device__ __forceinline__ uint64_t desc(uint32_t addr)
 // kind::tf32: FP32 accumulator (bits 4-5 = 1), A and B TF32 (bits 7-9 and
 // 10-12 = 2), K-major, N >> 3 at bits 17-22, M >> 4 at bits 24-28
 template<int V>
-constexpr uint32_t idesc()
+constexpr uint32_t idesc(int words = 1)
 {
-    return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t) (shape<V>::N >> 3) << 17) |
+    return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t) (words * shape<V>::N >> 3) << 17) |
         ((uint32_t) (M >> 4) << 24);
 }
 
@@ -84,8 +86,18 @@ __device__ __forceinline__ float tf32_hi(float x)
     return __uint_as_float((u + 0x1000u) & 0xFFFFE000u);
 }
 
+// x rounded to the nearest multiple of 2^-8 of the leading power of two of
+// `largest` (magic: grid_magic of it), |x| <= largest: at most 10 bits, a
+// TF32 number. x - on_grid(x) is exact.
+__device__ __forceinline__ float grid_magic(float largest)
+{
+    const uint32_t e = min(__float_as_uint(largest) & 0x7f800000u, 239u << 23);
+    return __uint_as_float((e + (15u << 23)) | 0x400000u);
+}
+__device__ __forceinline__ float on_grid(float x, float magic) { return __fadd_rn(__fadd_rn(x, magic), -magic); }
+
 struct ctx {
-    uint32_t a_hi, a_lo, b_hi, b_lo, b_dl;
+    uint32_t a_hi, a_lo, b_hi, b_lo, b_dl, a_fix, b_fix;
     float* rows;  // the A_hi region as plain rows of V floats (mixed tiles)
     uint32_t tmem;
     uint32_t mbar;
@@ -160,19 +172,25 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16])
 // Bdl correction. The second accumulator takes B_rest (D1 = A_hi B_rest).
 // Rows n >= V and columns k >= V are zero. Called by all threads; a barrier
 // must follow.
-// (bd, bdl: V x V, rows ld apart.)
-template<int V>
-__device__ __forceinline__ void stage_b(const ctx& c, const float* bd, const float* bdl, int ld)
+// (bd, bdl: V x V, rows ld apart.) FIX: B_fix takes the entries on the grid of
+// the largest, bmax, and the three words above what is left of them.
+template<int V, bool FIX = false>
+__device__ __forceinline__ void stage_b(const ctx& c, const float* bd, const float* bdl, int ld, float bmax = 0.0f)
 {
     using S = shape<V>;
+    const float magic = grid_magic(bmax);
     for (int e = threadIdx.x; e < S::N * S::KC; e += M) {
         const int n = e / S::KC, kc = e % S::KC;
-        float h[4], l[4], dl[4];
+        float h[4], l[4], dl[4], f[4];
 #pragma unroll
         for (int q = 0; q < 4; q++) {
             const int k = kc * 4 + q;
             const bool in = n < V && k < V;
-            const float b = in ? bd[n * ld + k] : 0.0f;
+            float b = in ? bd[n * ld + k] : 0.0f;
+            if constexpr (FIX) {
+                f[q] = on_grid(b, magic);
+                b -= f[q];                      // exact
+            }
             h[q] = tf32_hi(b);
             const float r = b - h[q];           // exact
             l[q] = tf32_hi(r);
@@ -182,6 +200,7 @@ __device__ __forceinline__ void stage_b(const ctx& c, const float* bd, const flo
         st16(c.b_hi + o, h[0], h[1], h[2], h[3]);
         st16(c.b_lo + o, l[0], l[1], l[2], l[3]);
         st16(c.b_dl + o, dl[0], dl[1], dl[2], dl[3]);
+        if constexpr (FIX) st16(c.b_fix + o, f[0], f[1], f[2], f[3]);
     }
 }
 
@@ -212,12 +231,55 @@ __device__ __forceinline__ void write_row(const ctx& c, const float (&x)[V])
     });
 }
 
-// D0 = A_hi Bhi^T + A_hi Blo^T + A_lo Bhi^T, D1 = A_hi Bdl^T: issued by
-// product_issue (all threads of the CTA, after write_row), complete after
-// product_wait. A wait that runs out is noted in *fail; the CTA then goes
+// The same row in three words: on the grid of its largest entry, then high
+// and low TF32 parts of the rest. The tensor cores truncate a sum to the
+// accumulator's 24 bits at every MMA; in D0 of the split above that is a bias
+// of about 3 x 2^-24 of the product towards zero, the same in every step (a
+// 6-level run of 500 points: error against 64 bits after 2,000 steps 5e-7,
+// 4 levels 2.1e-6; the FP32 FMA chain's rounding errors average out, 6e-8 and
+// 8e-8). The grid words' products are multiples of one unit and their sums
+// stay below 2^24 of it (36 x 2^9 x 2^9), so D0 is exact, and what D1's
+// truncation loses is 2^-9 as much: below the FMA chain's error (the same
+// runs: 6e-8 and 8e-8).
+template<int V>
+__device__ __forceinline__ void write_row_fix(const ctx& c, const float (&x)[V])
+{
+    using S = shape<V>;
+    const int row = threadIdx.x;
+    float largest = 0.0f;
+#pragma unroll
+    for (int k = 0; k < V; k++) largest = fmaxf(largest, fabsf(x[k]));
+    const float magic = grid_magic(largest);
+    static_for<0, S::KC>([&](auto KCI) {
+        constexpr int kc = decltype(KCI)::value;
+        float f[4], h[4], l[4];
+        static_for<0, 4>([&](auto QI) {
+            constexpr int q = decltype(QI)::value;
+            constexpr int k = kc * 4 + q;
+            if constexpr (k < V) {
+                f[q] = on_grid(x[k], magic);
+                const float y = x[k] - f[q];
+                h[q] = tf32_hi(y);
+                l[q] = tf32_hi(y - h[q]);
+            } else {
+                f[q] = h[q] = l[q] = 0.0f;
+            }
+        });
+        const uint32_t o = chunk<V>(row, kc);
+        st16(c.a_fix + o, f[0], f[1], f[2], f[3]);
+        st16(c.a_hi + o, h[0], h[1], h[2], h[3]);
+        st16(c.a_lo + o, l[0], l[1], l[2], l[3]);
+    });
+}
+
+// D0 = A_hi Bhi^T + A_hi Blo^T + A_lo Bhi^T, D1 = A_hi Bdl^T. FIX: with the
+// words in falling order, accumulator q (columns q N ..) takes the products
+// of word i of A and word q - i of B, q < 4.
+// Issued by product_issue (all threads of the CTA, after write_row),
+// complete after product_wait. A wait that runs out is noted in *fail; the CTA then goes
 // through its remaining steps without products or waits (its results are
 // void; every thread keeps meeting the same barriers).
-template<int V>
+template<int V, bool FIX = false>
 __device__ __forceinline__ void product_issue(const ctx& c)
 {
     using S = shape<V>;
@@ -231,6 +293,17 @@ __device__ __forceinline__ void product_issue(const ctx& c)
 #pragma unroll
         for (int ks = 0; ks < S::K / 8; ks++) {
             const uint32_t o = (uint32_t) ks * 256u;
+            if constexpr (FIX) {
+                // the words of B lie one after the other: one MMA takes several
+                // (an MMA of 48 columns takes as long as one of 192; with one
+                // per pair of words, 50 a step, a 6-level step of 65,536
+                // points took 36.1 us, with these 15 it takes 21.9)
+                const uint64_t b = desc<V>(c.b_fix + o);
+                mma_tf32(c.tmem, desc<V>(c.a_fix + o), b, idesc<V>(4), ks > 0 ? 1u : 0u);
+                mma_tf32(c.tmem + S::N, desc<V>(c.a_hi + o), b, idesc<V>(3), 1u);
+                mma_tf32(c.tmem + 2u * S::N, desc<V>(c.a_lo + o), b, idesc<V>(2), 1u);
+                continue;
+            }
             mma_tf32(c.tmem, desc<V>(c.a_hi + o), desc<V>(c.b_hi + o), id, ks > 0 ? 1u : 0u);
             mma_tf32(c.tmem, desc<V>(c.a_hi + o), desc<V>(c.b_lo + o), id, 1u);
             mma_tf32(c.tmem, desc<V>(c.a_lo + o), desc<V>(c.b_hi + o), id, 1u);
@@ -254,18 +327,30 @@ __device__ __forceinline__ bool product_wait(ctx& c)
     return all;
 }
 
-// Row threadIdx.x of D0 and D1, 16 columns at a time: f(i, D0[i], D1[i])
-// for i < V (i a compile-time constant).
-template<int V, class F>
+// Row threadIdx.x of D0 and D1 (FIX: of D0 and of the sum of the others), 16
+// columns at a time: f(i, D0[i], D1[i]) for i < V (i a compile-time constant).
+template<int V, bool FIX = false, class F>
 __device__ __forceinline__ void consume_row(const ctx& c, F&& f)
 {
+    constexpr uint32_t next = FIX ? (uint32_t) shape<V>::N : D1_COL;
     const uint32_t lane = (uint32_t) ((threadIdx.x >> 5) * 32) << 16;
     static_for<0, (V + 15) / 16>([&](auto BI) {
         constexpr int b = decltype(BI)::value;
-        float v[16], w[16];
+        float v[16], w[16], low[16];
+        if constexpr (FIX) {
+            tmem_ld16(c.tmem + lane + 3u * next + (uint32_t) (b * 16), low);
+            tmem_ld16(c.tmem + lane + 2u * next + (uint32_t) (b * 16), w);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+            for (int q = 0; q < 16; q++) low[q] += w[q];
+        }
         tmem_ld16(c.tmem + lane + (uint32_t) (b * 16), v);
-        tmem_ld16(c.tmem + lane + D1_COL + (uint32_t) (b * 16), w);
+        tmem_ld16(c.tmem + lane + next + (uint32_t) (b * 16), w);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        if constexpr (FIX) {
+#pragma unroll
+            for (int q = 0; q < 16; q++) w[q] += low[q];
+        }
         static_for<0, 16>([&](auto QI) {
             constexpr int q = decltype(QI)::value;
             if constexpr (b * 16 + q < V) f(std::integral_constant<int, b * 16 + q>{}, v[q], w[q]);
@@ -336,24 +421,26 @@ __device__ __forceinline__ void cvr_update_df_tc(
 // (the N^2 x N^2 matrix and its low words: 2 N^4 of the step's FMAs, each
 // with a coefficient from shared memory) on the tensor cores. The product
 // needs only the state before the step, so its MMAs run while the CUDA cores
-// solve for the field-dependent part. One 6-level run of 65,536 points: 34.4
-// -> 21.5 us a step, what is left being the solve and its products on 8
-// warps per SM (255 registers).
+// solve for the field-dependent part. Runs of 65,536 points, us a step, CUDA
+// cores / this form: 4 levels 6.54 / 6.26, 5 levels 14.3 / 12.8, 6 levels
+// 33.5 / 21.9; what is left at 6 is the solve and its products on 8 warps per
+// SM (255 registers).
 template<int N>
 __device__ __forceinline__ void cayley_update_df_tc(
     ctx& c, float (&rh)[N * N], float (&rl)[N * N], float e, float& pout, const float* cf)
 {
     constexpr int NN = N * N;
     const pre::cay_layout L = pre::make_cay_layout(N);
-    write_row<NN>(c, rh);
-    product_issue<NN>(c);
+    write_row_fix<NN>(c, rh);
+    product_issue<NN, true>(c);
     float inc[NN];
     cayley_increment_df<N>(rh, e, cf, inc);
     if (!product_wait(c)) return;
     float acc = 0.0f;
-    consume_row<NN>(c, [&](auto I, float d, float dl) {
+    consume_row<NN, true>(c, [&](auto I, float d, float dl) {
         constexpr int i = decltype(I)::value;
-        df_acc(rh[i], rl[i], inc[i] + d, dl);
+        const float v = d + dl;  // |dl| < |d|, or d = 0
+        df_acc(rh[i], rl[i], inc[i] + v, (d - v) + dl);
         df_renorm(rh[i], rl[i]);
         acc = fmaf(cf[L.gP + i], rh[i], fmaf(cf[L.gP + i], rl[i], acc));
     });

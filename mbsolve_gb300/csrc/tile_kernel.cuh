@@ -630,12 +630,13 @@ struct tc_res {
     int* fail;        // shared: a completion wait ran out
 };
 
+template<uint32_t COLS>
 __device__ __forceinline__ tc_res tc_acquire(uint32_t* tmem_sh, uint64_t* mbar, uint32_t* phase_sh, int* fail_sh)
 {
     if (threadIdx.x < 32) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                          (uint32_t) __cvta_generic_to_shared(tmem_sh)),
-                     "r"(tc::TMEM_COLS)
+                     "r"(COLS)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -653,6 +654,7 @@ __device__ __forceinline__ tc_res tc_acquire(uint32_t* tmem_sh, uint64_t* mbar, 
     return tc_res{ *tmem_sh, (uint32_t) __cvta_generic_to_shared(mbar), phase_sh, fail_sh };
 }
 
+template<uint32_t COLS>
 __device__ __forceinline__ void tc_release(const tc_res& r)
 {
     tc::fence_before();
@@ -666,7 +668,7 @@ __device__ __forceinline__ void tc_release(const tc_res& r)
         }
         __syncwarp();
         tc::fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(r.tmem), "r"(tc::TMEM_COLS)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(r.tmem), "r"(COLS)
                      : "memory");
     }
 }
@@ -824,7 +826,9 @@ __device__ __forceinline__ void step_body(const kparams<T>& p, uint32_t tile, ui
         using TS = tc::shape<D>;
         tcc.a_hi = ops;
         tcc.a_lo = ops + TS::A_BYTES;
-        tcc.b_hi = ops + 2u * TS::A_BYTES;
+        tcc.a_fix = ops + 2u * TS::A_BYTES;  // (the Cayley form's)
+        tcc.b_fix = ops + 3u * TS::A_BYTES;
+        tcc.b_hi = ALGO == 2 ? tcc.b_fix + TS::B_BYTES : ops + 2u * TS::A_BYTES;
         tcc.b_lo = tcc.b_hi + TS::B_BYTES;
         tcc.b_dl = tcc.b_lo + TS::B_BYTES;
         tcc.tmem = res.tmem;
@@ -838,7 +842,7 @@ __device__ __forceinline__ void step_body(const kparams<T>& p, uint32_t tile, ui
                 tc::stage_b<D>(tcc, mat + pre::FDTD_END, mat + pre::FDTD_END + D * D, D);
             } else {
                 const pre::cay_layout L = pre::make_cay_layout(LEV);
-                tc::stage_b<D>(tcc, mat + L.B0, mat + L.B0l, L.NP);
+                tc::stage_b<D, true>(tcc, mat + L.B0, mat + L.B0l, L.NP, mat[L.maxB0]);
             }
         }
     }
@@ -970,9 +974,10 @@ __global__ void __launch_bounds__(tc::M, tc_blocks(ALGO, LEV)) step_kernel_tc(co
     __shared__ __align__(8) uint64_t mbar[2];
     __shared__ uint32_t tmem_sh, phase_sh;
     __shared__ int fail_sh;
-    const tc_res r = tc_acquire(&tmem_sh, mbar, &phase_sh, &fail_sh);
+    constexpr uint32_t COLS = tc::shape<density_len<ALGO, LEV>::value, ALGO == 2>::TMEM_COLS;
+    const tc_res r = tc_acquire<COLS>(&tmem_sh, mbar, &phase_sh, &fail_sh);
     step_body<float, ALGO, LEV, 1, tc::M, true>(p, blockIdx.x, p.launch_idx, false, r);
-    tc_release(r);
+    tc_release<COLS>(r);
 }
 
 // 2-level FP32 kernels with bulk-copy (TMA) staging of the tile state; not
@@ -1073,9 +1078,10 @@ __global__ void __launch_bounds__(tc::M, tc_blocks(ALGO, LEV))
     __shared__ __align__(8) uint64_t mbar[2];
     __shared__ uint32_t tmem_sh, phase_sh;
     __shared__ int fail_sh;
-    const tc_res r = tc_acquire(&tmem_sh, mbar, &phase_sh, &fail_sh);
+    constexpr uint32_t COLS = tc::shape<density_len<ALGO, LEV>::value, ALGO == 2>::TMEM_COLS;
+    const tc_res r = tc_acquire<COLS>(&tmem_sh, mbar, &phase_sh, &fail_sh);
     persist_loop<float, ALGO, LEV, 1, tc::M, true>(p, q, r);
-    tc_release(r);
+    tc_release<COLS>(r);
 }
 
 }  // namespace mbg
