@@ -38,16 +38,16 @@ std::vector<kernel_entry<T> >& kernel_registry()
 }
 
 template<typename T>
-bool register_kernel(int algo, int lev, int C, int NT, launch_fn<T> fn, int staging, persist_fn<T> pfn)
+bool register_kernel(int algo, int lev, int C, int NT, launch_fn<T> fn, int staging, persist_fn<T> pfn, int medium)
 {
-    kernel_registry<T>().push_back(kernel_entry<T>{ algo, lev, C, NT, fn, staging, pfn });
+    kernel_registry<T>().push_back(kernel_entry<T>{ algo, lev, C, NT, fn, staging, pfn, medium });
     return true;
 }
 
 template std::vector<kernel_entry<float> >& kernel_registry<float>();
 template std::vector<kernel_entry<double> >& kernel_registry<double>();
-template bool register_kernel<float>(int, int, int, int, launch_fn<float>, int, persist_fn<float>);
-template bool register_kernel<double>(int, int, int, int, launch_fn<double>, int, persist_fn<double>);
+template bool register_kernel<float>(int, int, int, int, launch_fn<float>, int, persist_fn<float>, int);
+template bool register_kernel<double>(int, int, int, int, launch_fn<double>, int, persist_fn<double>, int);
 
 // -------------------------------------------------------------- names
 
@@ -1245,6 +1245,20 @@ private:
         MBG_CK(cudaStreamSynchronize(stream_));
     }
 
+    // whether every medium's Hamiltonian is diagonal
+    bool diagonal_media() const
+    {
+        for (const auto& r : runs_)
+            for (const pre::mat_in& m : r.mats)
+                for (int i = 0; i < m.N * m.N; i++)
+                    if (i % (m.N + 1) != 0 && (m.h_re[i] != 0.0 || m.h_im[i] != 0.0)) return false;
+        return true;
+    }
+    bool fits(const kernel_entry<T>& e) const
+    {
+        return e.medium == MEDIUM_ANY || (e.medium == MEDIUM_DIAG) == diagonal_;
+    }
+
     static int align_halo(int depth) { return (depth + 7) & ~7; }
     // a run of a single point has no neighbours
     int tile_halo(int depth) const { return staging_ == STAGING_POINT ? 0 : align_halo(depth); }
@@ -1291,17 +1305,15 @@ private:
     launch_fn<T> find_kernel(int C, int NT) const
     {
         for (const auto& e : kernel_registry<T>())
-            if (e.algo == kind_.algo && e.lev == kind_.N && e.C == C && e.NT == NT && e.staging == staging_ && e.fn)
+            if (e.algo == kind_.algo && e.lev == kind_.N && e.C == C && e.NT == NT && e.staging == staging_ && fits(e))
                 return e.fn;
         return nullptr;
     }
 
-    // a shape may be registered twice (its persistent kernel compiled in a
-    // translation unit of its own): the first entry with one
     persist_fn<T> find_persistent(int C, int NT) const
     {
         for (const auto& e : kernel_registry<T>())
-            if (e.algo == kind_.algo && e.lev == kind_.N && e.C == C && e.NT == NT && e.staging == 0 && e.pfn)
+            if (e.algo == kind_.algo && e.lev == kind_.N && e.C == C && e.NT == NT && e.staging == 0 && fits(e))
                 return e.pfn;
         return nullptr;
     }
@@ -1329,6 +1341,7 @@ private:
     }
 
     int staging_ = 0;
+    bool diagonal_ = false;  // diagonal_media()
 
     kparams<T> params(int in, uint32_t launch_idx, uint32_t nsub, bool record, const unsigned long long* step) const
     {
@@ -1614,6 +1627,7 @@ private:
     void choose_tuning(const mbg_tuning* user)
     {
         staging_ = 0;
+        diagonal_ = diagonal_media();
         if (staging_wanted() || (user && user->staging == 1))
             for (const auto& e : kernel_registry<T>())
                 if (e.algo == kind_.algo && e.lev == kind_.N && e.staging == 1) staging_ = 1;
@@ -1667,7 +1681,7 @@ private:
                 const bool joint = cells_ <= (1u << 17);
                 std::vector<std::pair<tuning, double> > shapes;
                 for (const auto& e : kernel_registry<T>()) {
-                    if (e.algo != kind_.algo || e.lev != kind_.N || e.staging != staging_ || !e.fn) continue;
+                    if (e.algo != kind_.algo || e.lev != kind_.N || e.staging != staging_ || !fits(e)) continue;
                     for (int d : depth_list) {
                         tuning c = t;
                         c.C = e.C;

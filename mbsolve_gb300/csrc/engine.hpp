@@ -131,6 +131,12 @@ void launch_precompute(
 // kernels of runs of a single grid point (point_cayley.cuh).
 enum : int { STAGING_REGS = 0, STAGING_BULK = 1, STAGING_POINT = 2 };
 
+// Values of kernel_entry::medium: what a kernel is for. DIAG: runs whose
+// Hamiltonians are all diagonal (block-diagonal field-free matrices of the
+// FP32 Cayley step), OTHER: the others. Two kernels of one launch shape
+// differ in it.
+enum : int { MEDIUM_ANY = 0, MEDIUM_DIAG = 1, MEDIUM_OTHER = 2 };
+
 // Kernel registry: every instantiated (algo, levels, C, NT) launcher.
 template<typename T>
 using launch_fn = void (*)(const kparams<T>&, unsigned grid, size_t smem, cudaStream_t s);
@@ -146,6 +152,7 @@ struct kernel_entry {
     launch_fn<T> fn;
     int staging;  // STAGING_*
     persist_fn<T> pfn;  // null where the shape has no persistent kernel
+    int medium;  // MEDIUM_*
 };
 
 template<typename T>
@@ -153,6 +160,6 @@ std::vector<kernel_entry<T> >& kernel_registry();
 
 template<typename T>
 bool register_kernel(int algo, int lev, int C, int NT, launch_fn<T> fn, int staging = 0,
-                     persist_fn<T> pfn = nullptr);
+                     persist_fn<T> pfn = nullptr, int medium = MEDIUM_ANY);
 
 }  // namespace mbg

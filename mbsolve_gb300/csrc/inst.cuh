@@ -120,14 +120,14 @@ unsigned launch_persist_tc(const kparams<float>& p, const persist_params& q, siz
 }  // namespace mbg
 
 // with a persistent kernel as well
-#define MBG_REG_TC_P(ALGO, LEV)                                                    \
+#define MBG_REG_TC_P(ALGO, LEV, MEDIUM)                                            \
     static const bool MBG_CAT(mbg_reg_, __LINE__) = ::mbg::register_kernel<float>( \
         ::mbg::ALGO, LEV, 1, ::mbg::tc::M, &::mbg::launch_step_tc<::mbg::ALGO, LEV>, 0, \
-        &::mbg::launch_persist_tc<::mbg::ALGO, LEV>);
-#define MBG_REG_CAY_P(T, LEV, C, NT)                                           \
+        &::mbg::launch_persist_tc<::mbg::ALGO, LEV>, ::mbg::MEDIUM);
+#define MBG_REG_CAY_P(T, LEV, C, NT, MEDIUM)                                   \
     static const bool MBG_CAT(mbg_reg_, __LINE__) = ::mbg::register_kernel<T>( \
         ::mbg::ALGO_CAYLEY, LEV, C, NT, &::mbg::launch_step<T, 2, LEV, C, NT>, 0, \
-        &::mbg::launch_persist<T, 2, LEV, C, NT>);
+        &::mbg::launch_persist<T, 2, LEV, C, NT>, ::mbg::MEDIUM);
 #define MBG_REG_CVR_P(T, LEV, C, NT)                                           \
     static const bool MBG_CAT(mbg_reg_, __LINE__) = ::mbg::register_kernel<T>( \
         ::mbg::ALGO_CVR, LEV, C, NT, &::mbg::launch_step<T, 1, LEV, C, NT>, 0,  \
