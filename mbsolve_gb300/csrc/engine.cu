@@ -1254,6 +1254,16 @@ private:
                     if (i % (m.N + 1) != 0 && (m.h_re[i] != 0.0 || m.h_im[i] != 0.0)) return false;
         return true;
     }
+    // and dipole operator real (with diagonal Hamiltonians: the zeros of
+    // cvr2_sparse at 2 levels)
+    bool real_dipoles() const
+    {
+        for (const auto& r : runs_)
+            for (const pre::mat_in& m : r.mats)
+                for (int i = 0; i < m.N * m.N; i++)
+                    if (m.mu_im[i] != 0.0) return false;
+        return true;
+    }
     bool fits(const kernel_entry<T>& e) const
     {
         return e.medium == MEDIUM_ANY || (e.medium == MEDIUM_DIAG) == diagonal_;
@@ -1483,7 +1493,17 @@ private:
 
     // ------------------------------------------------------ autotuner
 
-    std::string tune_key() const
+    // What decides between the candidates of a (GPU, solver): the media
+    // (which kernels fit, and which products a kernel skips), the size (by
+    // factors of two where shape and depth are tuned together, see
+    // choose_tuning; 16,384 2-level points take another pair than 100),
+    // the runs, and whether a persistent kernel is asked for. TUNE_SET
+    // changes with the set of kernels, so that a file's entries of another
+    // set are not read.
+    static constexpr const char* TUNE_SET = "k2";
+    static constexpr uint64_t JOINT_CELLS = 1u << 17;
+
+    std::string tune_key(int forced) const
     {
         std::ostringstream s;
         int dev = 0;
@@ -1493,7 +1513,15 @@ private:
             s << "_" << prop.multiProcessorCount << ":";
         }
         s << kind_.algo << ":" << kind_.N << ":s" << staging_ << ":" << (kind_.fp64 ? 64 : 32) << ":"
-          << (cells_ >> 16) << ":" << runs_.size() << ":" << std::min<uint64_t>(nt_max_, 256);
+          << (diagonal_ ? real_dipoles() ? "r" : "d" : "n") << ":";
+        if (cells_ <= JOINT_CELLS) {
+            int bits = 0;
+            for (uint64_t c = cells_; c; c >>= 1) bits++;
+            s << "b" << bits;
+        } else {
+            s << (cells_ >> 16);
+        }
+        s << ":" << runs_.size() << ":" << std::min<uint64_t>(nt_max_, 256) << ":p" << forced << ":" << TUNE_SET;
         return s.str();
     }
 
@@ -1657,7 +1685,7 @@ private:
         const char* env = std::getenv("MBG_AUTOTUNE");
         const bool autotune = !explicit_all && staging_ != STAGING_POINT && !(env && env[0] == '0');
         if (autotune) {
-            std::string key = tune_key();
+            std::string key = tune_key(persistent_forced(user));
             bool cached = false;
             {
                 std::lock_guard<std::mutex> lk(g_tune_mutex);
@@ -1678,7 +1706,7 @@ private:
                 // best shape (each stage ends with a run-off of its close
                 // contenders)
                 const int depth_list[] = { 1, 2, 4, 8, 16, 32, 64 };
-                const bool joint = cells_ <= (1u << 17);
+                const bool joint = cells_ <= JOINT_CELLS;
                 std::vector<std::pair<tuning, double> > shapes;
                 for (const auto& e : kernel_registry<T>()) {
                     if (e.algo != kind_.algo || e.lev != kind_.N || e.staging != staging_ || !fits(e)) continue;
