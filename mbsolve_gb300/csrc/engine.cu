@@ -1707,9 +1707,16 @@ private:
                 // contenders)
                 const int depth_list[] = { 1, 2, 4, 8, 16, 32, 64 };
                 const bool joint = cells_ <= JOINT_CELLS;
+                // (a persistent kernel asked for: the shapes that have one,
+                // where any has)
                 std::vector<std::pair<tuning, double> > shapes;
+                bool persist = false;
+                if (staging_ == STAGING_REGS && persistent_forced(user) == 1)
+                    for (const auto& e : kernel_registry<T>())
+                        persist |= e.algo == kind_.algo && e.lev == kind_.N && fits(e) && e.pfn;
                 for (const auto& e : kernel_registry<T>()) {
                     if (e.algo != kind_.algo || e.lev != kind_.N || e.staging != staging_ || !fits(e)) continue;
+                    if (persist && !e.pfn) continue;
                     for (int d : depth_list) {
                         tuning c = t;
                         c.C = e.C;
