@@ -848,6 +848,20 @@ public:
         }
     }
 
+    // the pinned chunks, allocated on first use; false where the system has
+    // no pinned memory left (the copy then goes through pageable memory)
+    bool pinned()
+    {
+        if (!pin_ && cudaMallocHost((void**) &pin_, 2 * PIN_CHUNK * sizeof(T)) != cudaSuccess) {
+            cudaGetLastError();
+            pin_ = nullptr;
+            return false;
+        }
+        for (auto& e : pin_done_)
+            if (!e) MBG_CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        return true;
+    }
+
     // n device values to doubles on the host; the stream is idle. Large FP32
     // records come through two pinned chunks, one converted while the other
     // arrives: a pageable copy of the whole record into a vector wrote and
@@ -858,15 +872,17 @@ public:
         if constexpr (sizeof(T) == sizeof(double)) {
             MBG_CK(cudaMemcpy(out, src, n * sizeof(T), cudaMemcpyDeviceToHost));
         } else {
-            if (n <= PIN_MIN) {
+            // several threads may read results of one engine: the chunks are
+            // one caller's at a time
+            std::unique_lock<std::mutex> lk(pin_mutex_, std::defer_lock);
+            if (n > PIN_MIN) lk.lock();
+            if (n <= PIN_MIN || !pinned()) {
+                if (lk) lk.unlock();
                 std::vector<T> tmp(n);
                 MBG_CK(cudaMemcpy(tmp.data(), src, n * sizeof(T), cudaMemcpyDeviceToHost));
                 for (uint64_t i = 0; i < n; i++) out[i] = (double) tmp[i];
                 return;
             }
-            if (!pin_) MBG_CK(cudaMallocHost((void**) &pin_, 2 * PIN_CHUNK * sizeof(T)));
-            for (auto& e : pin_done_)
-                if (!e) MBG_CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
             const uint64_t chunks = (n + PIN_CHUNK - 1) / PIN_CHUNK;
             auto count = [&](uint64_t k) { return std::min<uint64_t>(PIN_CHUNK, n - k * PIN_CHUNK); };
             auto fetch = [&](uint64_t k) {
@@ -964,6 +980,7 @@ private:
     cudaEvent_t region_[2] = { nullptr, nullptr };
     // copy_values: two pinned chunks, from the first large record on
     static constexpr uint64_t PIN_MIN = 1u << 15, PIN_CHUNK = 1u << 18;
+    std::mutex pin_mutex_;
     T* pin_ = nullptr;
     cudaEvent_t pin_done_[2] = { nullptr, nullptr };
 
