@@ -20,6 +20,7 @@ pre-activations [B, S, W] FP32, spectra Vh [B, 2 Mo, W] FP32 (Re modes then
 Im modes), mixed spectra Y [B, Mo, 2 W] FP32, mode blocks [Mo, 2W, 2W] BF16.
 """
 import math
+import threading
 
 import numpy as np
 import torch
@@ -113,6 +114,10 @@ class FNO:
         self._bufs = {}
         self._ibufs = {}
         self._progs = {}
+        # buffers, weight forms and programs are made by one thread at a time:
+        # a program holds the addresses of the buffers its results are read
+        # from
+        self._making = threading.RLock()
         self._blk_valid = False   # blk: BF16 mode blocks of the weights
         self._dense_valid = False  # _wb, _img: what infer() reads besides
         self._wb = {}   # BF16 copies of the dense weights (inference)
@@ -122,7 +127,12 @@ class FNO:
         # a copy lays its own programs out: they hold device addresses
         d = self.__dict__.copy()
         d["_progs"] = {}
+        del d["_making"]
         return d
+
+    def __setstate__(self, d):
+        self.__dict__.update(d)
+        self._making = threading.RLock()
 
     # ------------------------------------------------------------ helpers
     def _issue(self, key, calls, **inputs):
@@ -132,14 +142,15 @@ class FNO:
         if self.dev.type != "cuda":
             calls(**inputs)
             return
-        prog = self._progs.get(key)
-        if prog is None:
-            prog = K.Program()
-            for name, t in inputs.items():
-                prog.input(name, t)
-            with prog:
-                calls(**inputs)
-            self._progs[key] = prog
+        with self._making:
+            prog = self._progs.get(key)
+            if prog is None:
+                prog = K.Program()
+                for name, t in inputs.items():
+                    prog.input(name, t)
+                with prog:
+                    calls(**inputs)
+                self._progs[key] = prog
         prog.run(**inputs)
 
     def _views(self, flat):
@@ -181,14 +192,15 @@ class FNO:
     def _weights(self, infer):
         """Brings the BF16 forms of the weights up to date: the mode blocks,
         and what only infer() reads."""
-        if not self._blk_valid:
-            self._issue("blk", self._mode_blocks)
-            self._blk_valid = True
-        if infer and not self._dense_valid:
-            if self.fused_ok() and "G" not in self._img:
-                self._basis_images()
-            self._issue("dense", self._dense_weights)
-            self._dense_valid = True
+        with self._making:
+            if not self._blk_valid:
+                self._issue("blk", self._mode_blocks)
+                self._blk_valid = True
+            if infer and not self._dense_valid:
+                if self.fused_ok() and "G" not in self._img:
+                    self._basis_images()
+                self._issue("dense", self._dense_weights)
+                self._dense_valid = True
 
     def _mode_blocks(self):
         for l in range(self.sh.L):

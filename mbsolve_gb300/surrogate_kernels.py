@@ -37,6 +37,7 @@ class Program:
     The tensors of the recorded calls must outlive the program and stay where
     they are, except those given to input(), which stand for the tensor
     passed to run() under that name: same size, dtype and device, contiguous.
+    Several threads may run() one program, each with its own inputs.
     """
 
     _local = threading.local()
@@ -44,6 +45,7 @@ class Program:
     def __init__(self):
         self._ops, self._keep, self._inputs, self._patch = [], [], {}, []
         self._array = None
+        self._running = threading.Lock()  # run() writes into _array
 
     def input(self, name, t):
         self._inputs[name] = t
@@ -99,13 +101,15 @@ class Program:
             if (t.shape, t.dtype, t.device) != want or not t.is_contiguous():
                 raise ValueError("%s: need a contiguous tensor of %s, %s, %s"
                                  % ((name,) + want))
-        for name, where, (attr, k), off in self._patch:
-            a = inputs[name].data_ptr() + off
-            if k is None:
-                setattr(where, attr, a)
-            else:
-                getattr(where, attr)[k] = a
-        _native.check(_lib().mbg_fno_run(self._array, len(self._ops), _stream()))
+        # (the native call releases the interpreter lock)
+        with self._running:
+            for name, where, (attr, k), off in self._patch:
+                a = inputs[name].data_ptr() + off
+                if k is None:
+                    setattr(where, attr, a)
+                else:
+                    getattr(where, attr)[k] = a
+            _native.check(_lib().mbg_fno_run(self._array, len(self._ops), _stream()))
 
 
 def _recording():
