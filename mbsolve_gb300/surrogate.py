@@ -124,15 +124,19 @@ class FNO:
         self._img = {}  # BF16 tile images for the fused layer kernel
 
     def __getstate__(self):
-        # a copy lays its own programs out: they hold device addresses
+        # a copy lays its own programs out (they hold device addresses) and
+        # takes its own views (pickled, each would become a tensor by itself)
         d = self.__dict__.copy()
         d["_progs"] = {}
-        del d["_making"]
+        for name in ("_making", "p", "g"):
+            del d[name]
         return d
 
     def __setstate__(self, d):
         self.__dict__.update(d)
         self._making = threading.RLock()
+        self.p = self._views(self.theta)
+        self.g = self._views(self.grad)
 
     # ------------------------------------------------------------ helpers
     def _issue(self, key, calls, **inputs):
