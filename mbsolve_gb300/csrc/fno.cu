@@ -15,7 +15,8 @@
 // otherwise a thread gathers a whole core matrix into registers (any
 // strides, FP32 or BF16, converted to BF16 on the way; 16-byte loads along
 // whichever dimension is contiguous, transposed in registers where that is
-// not K) while the MMAs of the block before run, and stores it into one of
+// not K; operands that allow neither by strips of one row or element by
+// element) while the MMAs of the block before run, and stores it into one of
 // two stages (the smaller footprint keeps four CTAs per SM for the short-K
 // products of training). One elected thread issues the MMAs;
 // tcgen05.commit arrives on the stage's mbarrier when they have read the
@@ -70,7 +71,8 @@ static_assert(BM * (BN + 1) * 4 <= STAGES_GATHER * lay<true>::STAGE_BYTES &&
 enum : int32_t {
     LD_ANY = 0,   // any strides: element by element
     LD_K = 1,     // K contiguous, every row's 8-element chunks 16-byte aligned
-    LD_ROWS = 2   // rows contiguous, every 8 rows of a K entry 16-byte aligned
+    LD_ROWS = 2,  // rows contiguous, every 8 rows of a K entry 16-byte aligned
+    LD_STRIP = 3  // rows contiguous, unaligned: a thread takes one row
 };
 struct seg_t {
     const void* a;
@@ -116,6 +118,128 @@ __device__ __forceinline__ float ld_elem(const void* base, int32_t type, int64_t
     return reinterpret_cast<const float*>(base)[off];
 }
 
+// Two K entries as a BF16 pair; an entry outside the operand (in0, in1) is 0.
+// No branches but these predicates, and the storage type known, so that the
+// loads of a whole part of a tile are in flight together.
+__device__ __forceinline__ uint32_t ld_pair(const float* b, int64_t sk, bool in0, bool in1)
+{
+    const float x = in0 ? __ldg(b) : 0.0f, y = in1 ? __ldg(b + sk) : 0.0f;
+    return pack_bf16(x, y);
+}
+__device__ __forceinline__ uint32_t ld_pair(const uint16_t* b, int64_t sk, bool in0, bool in1)
+{
+    const uint32_t x = in0 ? __ldg(b) : 0u, y = in1 ? __ldg(b + sk) : 0u;
+    return x | y << 16;
+}
+
+// 8 contiguous K entries at a 16-byte boundary
+__device__ __forceinline__ void ld_chunk(const float* b, uint32_t (&w)[4])
+{
+    const float4 x = __ldg(reinterpret_cast<const float4*>(b));
+    const float4 y = __ldg(reinterpret_cast<const float4*>(b) + 1);
+    w[0] = pack_bf16(x.x, x.y);
+    w[1] = pack_bf16(x.z, x.w);
+    w[2] = pack_bf16(y.x, y.y);
+    w[3] = pack_bf16(y.z, y.w);
+}
+__device__ __forceinline__ void ld_chunk(const uint16_t* b, uint32_t (&w)[4])
+{
+    const uint4 q = __ldg(reinterpret_cast<const uint4*>(b));
+    w[0] = q.x;
+    w[1] = q.y;
+    w[2] = q.z;
+    w[3] = q.w;
+}
+
+// a core matrix of any strides (b: its first entry); nr, nk: its rows and K
+// entries inside the operand
+template<typename E>
+__device__ __forceinline__ void gather_any(const E* b, int64_t sr, int64_t sk, int nr, int nk, uint32_t (&w)[8][4])
+{
+    if (sk == 1 && nk == 8) {
+        // (some rows of an operand with an odd row stride are aligned)
+#pragma unroll
+        for (int r = 0; r < 8; r++) {
+            const E* at = b + r * sr;
+            if (r < nr && (reinterpret_cast<uintptr_t>(at) & 15) == 0) {
+                ld_chunk(at, w[r]);
+            } else {
+#pragma unroll
+                for (int j = 0; j < 4; j++) w[r][j] = ld_pair(at + 2 * j, 1, r < nr, r < nr);
+            }
+        }
+    } else {
+#pragma unroll
+        for (int r = 0; r < 8; r++)
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                w[r][j] = ld_pair(b + r * sr + 2 * j * sk, sk, r < nr && 2 * j < nk, r < nr && 2 * j + 1 < nk);
+    }
+}
+
+// LD_STRIP: NC K groups (from k0 on) of one row
+template<typename E, int NC>
+__device__ __forceinline__ void strip_run(const E* b, int64_t sk, bool row, int nk, uint32_t (*w)[4])
+{
+#pragma unroll
+    for (int i = 0; i < NC; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int k = 8 * i + 2 * j;
+            w[i][j] = ld_pair(b + k * sk, sk, row && k < nk, row && k + 1 < nk);
+        }
+}
+
+template<int NC>
+__device__ __forceinline__ void strip_part(
+    const gemm_params& p, bool is_a, int z, int row, int rows, int k0, uint32_t (*w)[4])
+{
+    int s = 0;
+    if (p.nseg > 1 && k0 >= p.kstart[1]) s = 1;
+    if (p.nseg > 2 && k0 >= p.kstart[2]) s = 2;
+    const seg_t& g = p.seg[s];
+    const int kl = k0 - p.kstart[s];
+    const int64_t sk = is_a ? g.a_sk : g.b_sk;
+    const int64_t off =
+        (int64_t) z * (is_a ? g.a_sz : g.b_sz) + (int64_t) row * (is_a ? g.a_sm : g.b_sn) + (int64_t) kl * sk;
+    const void* base = is_a ? g.a : g.b;
+    if ((is_a ? g.a_type : g.b_type) == MBG_BF16)
+        strip_run<uint16_t, NC>(reinterpret_cast<const uint16_t*>(base) + off, sk, row < rows, g.k - kl, w);
+    else
+        strip_run<float, NC>(reinterpret_cast<const float*>(base) + off, sk, row < rows, g.k - kl, w);
+    if (g.neg && is_a) {  // negate the product: A only
+#pragma unroll
+        for (int i = 0; i < NC; i++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) w[i][j] ^= 0x80008000u;
+    }
+}
+
+// NC K groups of row `row`, from k0 on: in one run where a segment holds them
+// (or the end of the last), else group by group
+template<int NC>
+__device__ __forceinline__ void gather_strip(
+    const gemm_params& p, bool is_a, int z, int row, int rows, int k0, uint32_t (&w)[8][4])
+{
+    bool split = false;
+    if (p.nseg > 1) split |= k0 < p.kstart[1] && p.kstart[1] < k0 + 8 * NC;
+    if (p.nseg > 2) split |= k0 < p.kstart[2] && p.kstart[2] < k0 + 8 * NC;
+    if (!split) {
+        strip_part<NC>(p, is_a, z, row, rows, k0, w);
+    } else {
+#pragma unroll 1
+        for (int i = 0; i < NC; i++) {
+            uint32_t one[1][4];
+            strip_part<1>(p, is_a, z, row, rows, k0 + 8 * i, one);
+#pragma unroll
+            for (int q = 0; q < NC; q++)
+                if (q == i)
+#pragma unroll
+                    for (int j = 0; j < 4; j++) w[q][j] = one[0][j];
+        }
+    }
+}
+
 // One core matrix of an operand on the gather path: 8 rows (row0 ..) x 8
 // consecutive K entries (k0 ..), BF16, w[r] the 16 bytes of row r. All its
 // loads are 16 bytes wide where the operand is contiguous along K (LD_K: a
@@ -125,6 +249,7 @@ __device__ __forceinline__ float ld_elem(const void* base, int32_t type, int64_t
 // thread and K block, each with its own type and bounds test), the products
 // of a training step (batch 64) took 23 to 122 us each, now 15 to 35 (caches
 // cold); the step 3.14 -> 1.40 ms.
+template<bool LOOSE>
 __device__ __forceinline__ void gather_unit(
     const gemm_params& p, bool is_a, int z, int row0, int rows, int k0, uint32_t (&w)[8][4])
 {
@@ -148,28 +273,15 @@ __device__ __forceinline__ void gather_unit(
     const int nk = min(8, g.k - kl), nr = min(8, rows - row0);
     if (ld == LD_K && nk == 8) {
         if (type == MBG_BF16) {
-            const __nv_bfloat16* b = reinterpret_cast<const __nv_bfloat16*>(base) + off;
+            const uint16_t* b = reinterpret_cast<const uint16_t*>(base) + off;
 #pragma unroll
             for (int r = 0; r < 8; r++)
-                if (r < nr) {
-                    const uint4 q = __ldg(reinterpret_cast<const uint4*>(b + r * sr));
-                    w[r][0] = q.x;
-                    w[r][1] = q.y;
-                    w[r][2] = q.z;
-                    w[r][3] = q.w;
-                }
+                if (r < nr) ld_chunk(b + r * sr, w[r]);
         } else {
             const float* b = reinterpret_cast<const float*>(base) + off;
 #pragma unroll
             for (int r = 0; r < 8; r++)
-                if (r < nr) {
-                    const float4 x = __ldg(reinterpret_cast<const float4*>(b + r * sr));
-                    const float4 y = __ldg(reinterpret_cast<const float4*>(b + r * sr) + 1);
-                    w[r][0] = pack_bf16(x.x, x.y);
-                    w[r][1] = pack_bf16(x.z, x.w);
-                    w[r][2] = pack_bf16(y.x, y.y);
-                    w[r][3] = pack_bf16(y.z, y.w);
-                }
+                if (r < nr) ld_chunk(b + r * sr, w[r]);
         }
     } else if (ld == LD_ROWS && nr == 8) {
         if (type == MBG_BF16) {
@@ -209,7 +321,12 @@ __device__ __forceinline__ void gather_unit(
                 for (int r = 0; r < 8; r++) w[r][j] = pack_bf16(x[0][r], x[1][r]);
             }
         }
+    } else if (LOOSE && type == MBG_BF16) {
+        gather_any(reinterpret_cast<const uint16_t*>(base) + off, sr, sk, nr, nk, w);
+    } else if (LOOSE) {
+        gather_any(reinterpret_cast<const float*>(base) + off, sr, sk, nr, nk, w);
     } else {
+        // an edge of the operand
 #pragma unroll
         for (int r = 0; r < 8; r++) {
             if (r >= nr) continue;
@@ -288,13 +405,16 @@ __device__ __forceinline__ void unit_pos(int t, bool rows_first, int& rg, int& k
     }
 }
 
+__device__ __forceinline__ void store_row(uint32_t dst, const uint32_t (&w)[4])
+{
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3])
+                 : "memory");
+}
+
 __device__ __forceinline__ void store_unit(uint32_t dst, const uint32_t (&w)[8][4])
 {
 #pragma unroll
-    for (int r = 0; r < 8; r++)
-        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst + 16u * r), "r"(w[r][0]), "r"(w[r][1]),
-                     "r"(w[r][2]), "r"(w[r][3])
-                     : "memory");
+    for (int r = 0; r < 8; r++) store_row(dst + 16u * r, w[r]);
 }
 
 // the operands' core matrices of one K block held in registers between their
@@ -304,35 +424,64 @@ struct block_regs {
     uint32_t a[8][4], b[8][4];
 };
 static_assert((BM / 8) * (BK / 8) == NTH && (BN / 8) * (BK / 8) == NTH / 2, "one core matrix per thread");
+static_assert(BM == NTH && BN * 2 == NTH && BK == 64, "rows of a strip per thread");
 
-__device__ __forceinline__ bool rows_first(const gemm_params& p, bool is_a, int kb)
+// the form of the segment in which K block kb starts: it decides which part
+// of the tile a thread takes (a part in another segment is read in that one's)
+__device__ __forceinline__ int32_t block_form(const gemm_params& p, bool is_a, int kb)
 {
     const int k0 = kb * BK;
     int s = 0;
     if (p.nseg > 1 && k0 >= p.kstart[1]) s = 1;
     if (p.nseg > 2 && k0 >= p.kstart[2]) s = 2;
-    return (is_a ? p.seg[s].a_sm : p.seg[s].b_sn) == 1;
+    return is_a ? p.seg[s].a_ld : p.seg[s].b_ld;
 }
 
+// LD_STRIP: thread t takes row t of A (all of the block's K groups) and row t
+// mod 64 of B (half of them), so that the lanes of a load read 32 adjacent
+// rows. By core matrices a load's lanes lie 8 rows apart. FP32 products, us,
+// element by element / by core matrices / by rows: 1000 x 1001 x 999 125 / 199
+// / 50, 2000 x 2000 x 2000 354 / 467 / 118.
+template<bool LOOSE>
 __device__ __forceinline__ void load_block(const gemm_params& p, int z, int m0, int n0, int kb, block_regs& r)
 {
     int rg, kg;
-    unit_pos<BM / 8>(threadIdx.x, rows_first(p, true, kb), rg, kg);
-    gather_unit(p, true, z, m0 + rg * 8, p.m, kb * BK + kg * 8, r.a);
-    if (threadIdx.x < NTH / 2) {
-        unit_pos<BN / 8>(threadIdx.x, rows_first(p, false, kb), rg, kg);
-        gather_unit(p, false, z, n0 + rg * 8, p.n, kb * BK + kg * 8, r.b);
+    const int32_t fa = block_form(p, true, kb), fb = block_form(p, false, kb);
+    if (LOOSE && fa == LD_STRIP) {
+        gather_strip<8>(p, true, z, m0 + (int) threadIdx.x, p.m, kb * BK, r.a);
+    } else {
+        unit_pos<BM / 8>(threadIdx.x, fa == LD_ROWS, rg, kg);
+        gather_unit<LOOSE>(p, true, z, m0 + rg * 8, p.m, kb * BK + kg * 8, r.a);
+    }
+    if (LOOSE && fb == LD_STRIP) {
+        gather_strip<4>(p, false, z, n0 + (int) (threadIdx.x % BN), p.n, kb * BK + (int) (threadIdx.x / BN) * 32, r.b);
+    } else if (threadIdx.x < NTH / 2) {
+        unit_pos<BN / 8>(threadIdx.x, fb == LD_ROWS, rg, kg);
+        gather_unit<LOOSE>(p, false, z, n0 + rg * 8, p.n, kb * BK + kg * 8, r.b);
     }
 }
 
+template<bool LOOSE>
 __device__ __forceinline__ void store_block(const gemm_params& p, int kb, uint32_t sa, uint32_t sb, const block_regs& r)
 {
     using L = lay<true>;
     int rg, kg;
-    unit_pos<BM / 8>(threadIdx.x, rows_first(p, true, kb), rg, kg);
-    store_unit(sa + (uint32_t) rg * L::SBO + (uint32_t) kg * L::LBO, r.a);
-    if (threadIdx.x < NTH / 2) {
-        unit_pos<BN / 8>(threadIdx.x, rows_first(p, false, kb), rg, kg);
+    const int32_t fa = block_form(p, true, kb), fb = block_form(p, false, kb);
+    if (LOOSE && fa == LD_STRIP) {
+        const uint32_t at = sa + (threadIdx.x >> 3) * L::SBO + (threadIdx.x & 7) * 16u;
+#pragma unroll
+        for (int i = 0; i < 8; i++) store_row(at + (uint32_t) i * L::LBO, r.a[i]);
+    } else {
+        unit_pos<BM / 8>(threadIdx.x, fa == LD_ROWS, rg, kg);
+        store_unit(sa + (uint32_t) rg * L::SBO + (uint32_t) kg * L::LBO, r.a);
+    }
+    if (LOOSE && fb == LD_STRIP) {
+        const uint32_t row = threadIdx.x % BN, k4 = (threadIdx.x / BN) * 4u;
+        const uint32_t at = sb + (row >> 3) * L::SBO + (row & 7) * 16u + k4 * L::LBO;
+#pragma unroll
+        for (int i = 0; i < 4; i++) store_row(at + (uint32_t) i * L::LBO, r.b[i]);
+    } else if (threadIdx.x < NTH / 2) {
+        unit_pos<BN / 8>(threadIdx.x, fb == LD_ROWS, rg, kg);
         store_unit(sb + (uint32_t) rg * L::SBO + (uint32_t) kg * L::LBO, r.b);
     }
 }
@@ -344,7 +493,10 @@ __device__ __forceinline__ void red_add4(float* a, float4 v)
                  : "memory");
 }
 
-template<int STAGES, int AHEAD>
+// LOOSE: a gather-path operand is not LD_K or LD_ROWS (an instantiation of its
+// own: beside the loads of the others, even never taken, the aligned ones cost
+// 5 to 10 % more)
+template<int STAGES, int AHEAD, bool LOOSE = false>
 __global__ void __launch_bounds__(NTH) gemm_kernel(const gemm_params p)
 {
     constexpr bool GATHER = AHEAD == 0;  // only the asynchronous instantiations stage ahead
@@ -386,13 +538,13 @@ __global__ void __launch_bounds__(NTH) gemm_kernel(const gemm_params p)
     // stage block j: by asynchronous copies, or (gather path) from the
     // registers its loads went to while the MMAs of the block before ran
     block_regs regs;
-    if constexpr (GATHER) load_block(p, z, m0, n0, kb0, regs);
+    if constexpr (GATHER) load_block<LOOSE>(p, z, m0, n0, kb0, regs);
     auto stage = [&](int j) {
         const uint32_t sa = base + (uint32_t) (j % STAGES) * L::STAGE_BYTES;
         if constexpr (!GATHER)
             async_stage(p, z, m0, n0, kb0 + j, sa, sa + L::A_BYTES);
         else
-            store_block(p, kb0 + j, sa, sa + L::A_BYTES, regs);
+            store_block<LOOSE>(p, kb0 + j, sa, sa + L::A_BYTES, regs);
     };
     // exactly AHEAD copy groups before the loop (empty ones when there are
     // fewer blocks), so that waiting for all but the AHEAD most recent groups
@@ -430,7 +582,7 @@ __global__ void __launch_bounds__(NTH) gemm_kernel(const gemm_params p)
             mma_commit(mb0 + 8u * st);
         }
         if constexpr (GATHER)
-            if (it + 1 < nit) load_block(p, z, m0, n0, kb0 + it + 1, regs);
+            if (it + 1 < nit) load_block<LOOSE>(p, z, m0, n0, kb0 + it + 1, regs);
     }
     cp_async_wait<0>();  // no copy outlives the loop (a break leaves some in flight)
 
@@ -831,14 +983,15 @@ void require(bool c, const char* msg)
 // Whether the gather path can read an operand by 16-byte loads along K or
 // along its rows: that dimension contiguous, every other stride and the
 // base multiples of 16 bytes (a core matrix starts at a multiple of 8 rows
-// and, within its segment, of 8 K entries).
+// and, within its segment, of 8 K entries); if not, whether its rows are
+// adjacent.
 int32_t load_form(const void* base, int32_t type, int64_t sr, int64_t sk, int64_t sz)
 {
     const int64_t w = type == MBG_BF16 ? 8 : 4;
-    if ((reinterpret_cast<uintptr_t>(base) & 15) != 0 || sz % w != 0) return LD_ANY;
-    if (sk == 1 && sr % w == 0) return LD_K;
-    if (sr == 1 && sk % w == 0) return LD_ROWS;
-    return LD_ANY;
+    const bool aligned = (reinterpret_cast<uintptr_t>(base) & 15) == 0 && sz % w == 0;
+    if (aligned && sk == 1 && sr % w == 0) return LD_K;
+    if (aligned && sr == 1 && sk % w == 0) return LD_ROWS;
+    return sr == 1 ? LD_STRIP : LD_ANY;
 }
 
 void gemm(const mbg_gemm_desc* d, cudaStream_t s)
@@ -875,6 +1028,9 @@ void gemm(const mbg_gemm_desc* d, cudaStream_t s)
     }
     p.kstart[d->nseg] = kt;
     p.ktotal = kt;
+    bool loose = false;
+    for (int i = 0; i < d->nseg; i++)
+        for (const int32_t ld : { p.seg[i].a_ld, p.seg[i].b_ld }) loose |= ld == LD_ANY || ld == LD_STRIP;
     // asynchronous 16-byte copies need BF16 operands with K contiguous and
     // every row (and batch) start on a 16-byte boundary, and no negation
     bool async_ok = true;
@@ -939,6 +1095,8 @@ void gemm(const mbg_gemm_desc* d, cudaStream_t s)
                              lay<false>::smem(STAGES_ASYNC));
         cudaFuncSetAttribute(gemm_kernel<STAGES_GATHER, AHEAD_GATHER>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              lay<true>::smem(STAGES_GATHER));
+        cudaFuncSetAttribute(gemm_kernel<STAGES_GATHER, AHEAD_GATHER, true>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, lay<true>::smem(STAGES_GATHER));
         cudaFuncSetAttribute(gemm_kernel<STAGES_SHORT, AHEAD_SHORT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              lay<false>::smem(STAGES_SHORT));
     });
@@ -949,6 +1107,8 @@ void gemm(const mbg_gemm_desc* d, cudaStream_t s)
         gemm_kernel<STAGES_SHORT, AHEAD_SHORT><<<grid, NTH, lay<false>::smem(STAGES_SHORT), s>>>(p);
     else if (p.async_ok)
         gemm_kernel<STAGES_ASYNC, AHEAD_ASYNC><<<grid, NTH, lay<false>::smem(STAGES_ASYNC), s>>>(p);
+    else if (loose)
+        gemm_kernel<STAGES_GATHER, AHEAD_GATHER, true><<<grid, NTH, lay<true>::smem(STAGES_GATHER), s>>>(p);
     else
         gemm_kernel<STAGES_GATHER, AHEAD_GATHER><<<grid, NTH, lay<true>::smem(STAGES_GATHER), s>>>(p);
     check_launch("gemm_kernel");
