@@ -98,6 +98,10 @@ MBG_HD bool hasto_record(double ratio, uint64_t n)
     return last != next;
 }
 
+// the largest temporal depth (steps per launch): the kernels' step schedules
+// have this many entries
+constexpr int TILE_MAX_STEPS = 256;
+
 MBG_HD int cvr_len(int N) { return N * N - 1; }
 
 }  // namespace mbg

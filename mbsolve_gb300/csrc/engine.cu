@@ -566,7 +566,7 @@ struct dbuf {
 
 static const uint64_t GUARD_FRONT = 512;  // >= largest halo
 static const uint64_t GUARD_BACK = 8192;  // >= widest tile
-static const int MAX_DEPTH = 256;  // = TILE_MAX_STEPS of the kernels
+static const int MAX_DEPTH = TILE_MAX_STEPS;
 
 static std::mutex g_tune_mutex;
 static std::map<std::string, tuning> g_tune_cache;
@@ -574,7 +574,8 @@ static bool g_tune_file_read = false;
 
 // Autotuner results persist across processes in the file named by the
 // environment variable MBG_TUNE_CACHE, when it is set: one line
-// "key C NT depth graph" per tuned problem (keys contain the GPU's name).
+// "key C NT depth graph" per tuned problem (keys contain the GPU's name);
+// lines out of the engine's range are left out.
 // Called with g_tune_mutex held.
 static void tune_file_read()
 {
@@ -586,7 +587,7 @@ static void tune_file_read()
     std::string key;
     tuning t;
     while (f >> key >> t.C >> t.NT >> t.depth >> t.graph)
-        if (t.C > 0 && t.NT > 0 && t.depth > 0) g_tune_cache[key] = t;
+        if (t.C > 0 && t.NT > 0 && t.depth > 0 && t.depth <= MAX_DEPTH && t.graph > 0) g_tune_cache[key] = t;
 }
 
 static void tune_file_append(const std::string& key, const tuning& t)

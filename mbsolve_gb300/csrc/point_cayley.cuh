@@ -18,7 +18,6 @@
 namespace mbg {
 
 constexpr int POINT_THREADS = 32;
-constexpr int POINT_DEPTH = TILE_MAX_STEPS;
 
 // 1 / x by two Newton steps from an FP32 reciprocal (22 -> 44 -> 88 bits, the
 // last rounded to FP64: within an ulp): 4 FP64 instructions instead of a

@@ -22,7 +22,6 @@ struct density_len {
 // sources and records that touch one tile, gathered once per launch
 constexpr int TILE_MAX_SRC = 8;
 constexpr int TILE_MAX_REC = 8;
-constexpr int TILE_MAX_STEPS = 256;  // the largest temporal depth
 constexpr int TILE_SRC_VALUES = 256; // source values staged per launch
 
 struct no_coef {
