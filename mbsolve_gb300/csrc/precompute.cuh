@@ -433,6 +433,51 @@ MBG_HD int solve_partial_pivot(double* A, double* b, double* x, int n, const G& 
     return singular;
 }
 
+// The rotation J = [[c, s], [-s e^{-i phi}, c e^{-i phi}]] on (p, q) that
+// makes entry (p, q) of a Hermitian matrix vanish.
+struct jacobi_angle {
+    bool none;  // it is zero already
+    double c, s, ephr, ephi;
+    MBG_HD jacobi_angle(const double* are, const double* aim, int n, int p, int q)
+    {
+        const double zr = are[p * n + q], zi = aim[p * n + q];
+        const double app = are[p * n + p], aqq = are[q * n + q];
+        const double r = sqrt(zr * zr + zi * zi);
+        none = r == 0.0;
+        if (none) return;
+        ephr = zr / r;
+        ephi = zi / r;  // e^{i phi}
+        const double tau = (aqq - app) / (2.0 * r);
+        const double t = (tau >= 0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(1.0 + tau * tau));
+        c = 1.0 / sqrt(1.0 + t * t);
+        s = t * c;
+    }
+    // X <- X J, of one row
+    MBG_HD void columns(double* re, double* im, int p, int q) const
+    {
+        const double xpr = re[p], xpi = im[p], xqr = re[q], xqi = im[q];
+        // e^{-i phi} x_q
+        const double yr = ephr * xqr + ephi * xqi;
+        const double yi = ephr * xqi - ephi * xqr;
+        re[p] = c * xpr - s * yr;
+        im[p] = c * xpi - s * yi;
+        re[q] = s * xpr + c * yr;
+        im[q] = s * xpi + c * yi;
+    }
+    // X <- J^H X, of one column (entries p and q at P and Q)
+    MBG_HD void rows(double* re, double* im, int P, int Q) const
+    {
+        const double xpr = re[P], xpi = im[P], xqr = re[Q], xqi = im[Q];
+        // e^{+i phi} x_q
+        const double yr = ephr * xqr - ephi * xqi;
+        const double yi = ephr * xqi + ephi * xqr;
+        re[P] = c * xpr - s * yr;
+        im[P] = c * xpi - s * yi;
+        re[Q] = s * xpr + c * yr;
+        im[Q] = s * xpi + c * yi;
+    }
+};
+
 // Cyclic Jacobi eigen-decomposition of a complex Hermitian n x n matrix
 // (re/im row-major, overwritten; the diagonal ends as the eigenvalues).
 // Eigenvectors are the columns of (vre, vim). ws: 2 n doubles.
@@ -516,6 +561,46 @@ MBG_HD void jacobi_hermitian(
                     aim[q * n + k] = k == q || k == p ? 0.0 : s * xpi + c * yi;
                 }
                 g.sync();
+            }
+    }
+}
+
+// The same by one thread, a matrix's columns, its rows and the eigenvectors'
+// columns in loops of their own: the loops above, as a group of one, took
+// 2.13 s instead of 1.84 for 16,384 6-level materials (one thread each, at the
+// memory's rate) and 0.69 instead of 0.67 for 128.
+MBG_HD void jacobi_hermitian(
+    double* are,
+    double* aim,
+    double* vre,
+    double* vim,
+    int n,
+    double*,
+    const serial_group&)
+{
+    for (int i = 0; i < n * n; i++) {
+        vre[i] = (i % (n + 1) == 0) ? 1.0 : 0.0;
+        vim[i] = 0.0;
+    }
+    for (int sweep = 0; sweep < 60; sweep++) {
+        double off = 0.0, tot = 0.0;
+        for (int i = 0; i < n; i++)
+            for (int j = 0; j < n; j++) {
+                const double m2 = are[i * n + j] * are[i * n + j] + aim[i * n + j] * aim[i * n + j];
+                tot += m2;
+                if (i != j) off += m2;
+            }
+        if (off <= 1e-32 * tot) break;
+        for (int p = 0; p < n - 1; p++)
+            for (int q = p + 1; q < n; q++) {
+                const jacobi_angle a(are, aim, n, p, q);
+                if (a.none) continue;
+                for (int k = 0; k < n; k++) a.columns(are + k * n, aim + k * n, p, q);
+                for (int k = 0; k < n; k++) a.rows(are, aim, p * n + k, q * n + k);
+                are[p * n + q] = aim[p * n + q] = 0.0;
+                are[q * n + p] = aim[q * n + p] = 0.0;
+                aim[p * n + p] = aim[q * n + q] = 0.0;
+                for (int k = 0; k < n; k++) a.columns(vre + k * n, vim + k * n, p, q);
             }
     }
 }
