@@ -339,10 +339,21 @@ __global__ void precompute_kernel(
 // of it), the same for up to thousands side by side. A CTA of four warps
 // (one per FP64 unit) shares the matrix loops: 19 ms for 128 of them. It
 // loses where materials are small (2 levels: 3 x 3 loops) or so many that
-// the chip is full of them anyway.
+// one thread each fills the chip anyway. An ensemble's creation with n
+// materials, ms, thread / CTA, on both sides of the lines:
+//   cvr-rodr    3 levels: 1,024 11.7 / 7.4, 2,048 14.2 / 15.0
+//               4: 2,048 56 / 39, 4,096 65 / 75
+//               5: 4,096 223 / 178, 8,192 273 / 361
+//               6: 8,192 1,233 / 1,133, 16,384 1,838 / 2,229
+//   reg-cayley  3: 2,048 6.7 / 6.3, 4,096 to 16,384 within 4 %
+//               4: 2,048 7.5 / 6.6, 4,096 12.6 / 12.7
+//               5: 4,096 14.9 / 13.8, 8,192 25.6 / 26.4
+//               6: 8,192 31.0 / 29.8, 16,384 55 / 60
 bool block_precompute(int algo, int N, int n)
 {
-    return algo != ALGO_NOOP && N >= 3 && n <= 2048;
+    if (algo == ALGO_NOOP || N < 3) return false;
+    const int most = 1024 << (N - 3);
+    return n <= (algo == ALGO_CAYLEY ? std::max(most, 2048) : most);
 }
 
 void launch_precompute(
