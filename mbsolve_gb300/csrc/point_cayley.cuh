@@ -218,10 +218,12 @@ __global__ void __launch_bounds__(POINT_THREADS) point_cayley_kernel(const kpara
             if (!tl.overflow) {
                 if (kind >= 0 && (tl.due[t] >> lane & 1u)) {
                     const double v = value(kind, idx);
-                    if (left) *dst = v;
-                    left -= left ? 1 : 0;
+                    if (left) {
+                        *dst = v;
+                        if (!isfinite(v)) atomicOr(p.status, STATUS_NONFINITE);
+                        left--;
+                    }
                     dst++;
-                    if (!isfinite(v)) atomicOr(p.status, STATUS_NONFINITE);
                 }
             } else if (lane == 0) {
                 for_records(p, rd, tl, own, due, t, n, [](int, int) { return 0.0; },

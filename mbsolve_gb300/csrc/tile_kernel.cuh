@@ -252,10 +252,14 @@ __device__ __forceinline__ void for_records(const kparams<T>& p, const run_desc&
         if (todo & bit) {
             todo &= ~bit;
             const T v = field((own.rec >> 8) & 255, own.rec >> 16);
-            if (own.left) *own.dst = v;
-            own.left -= own.left ? 1u : 0u;
+            // (a step may be due beyond the last row; it is no part of the
+            // results)
+            if (own.left) {
+                *own.dst = v;
+                if (!isfinite(v)) atomicOr(p.status, STATUS_NONFINITE);
+                own.left--;
+            }
             own.dst++;
-            if (!isfinite(v)) atomicOr(p.status, STATUS_NONFINITE);
         }
         if (todo == 0u) return;
     }
