@@ -119,6 +119,7 @@ __global__ void __launch_bounds__(POINT_THREADS) point_cayley_kernel(const kpara
                 kind = 5;
             if (rc.type == REC_COH_IM && rc.row_idx > rc.col_idx) kind += 8;
         }
+        if (left == 0) kind = -1;  // steps due beyond the last row take none
     }
     auto shf = [&](double v, int src) { return __shfl_sync(ALL, v, src); };
     auto dissipate = [&](double& re, double& im) {
@@ -218,12 +219,9 @@ __global__ void __launch_bounds__(POINT_THREADS) point_cayley_kernel(const kpara
             if (!tl.overflow) {
                 if (kind >= 0 && (tl.due[t] >> lane & 1u)) {
                     const double v = value(kind, idx);
-                    if (left) {
-                        *dst = v;
-                        if (!isfinite(v)) atomicOr(p.status, STATUS_NONFINITE);
-                        left--;
-                    }
-                    dst++;
+                    *dst++ = v;
+                    if (--left == 0) kind = -1;
+                    if (!isfinite(v)) atomicOr(p.status, STATUS_NONFINITE);
                 }
             } else if (lane == 0) {
                 for_records(p, rd, tl, own, due, t, n, [](int, int) { return 0.0; },

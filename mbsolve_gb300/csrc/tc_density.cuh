@@ -104,6 +104,7 @@ struct ctx {
     uint32_t phase;
     uint32_t wait_limit;  // polls of a completion wait
     volatile int* fail;   // shared: a completion wait of this CTA ran out
+    bool live;            // none of this thread's did
 };
 
 __device__ __forceinline__ void mma_tf32(uint32_t d, uint64_t a, uint64_t b, uint32_t id, uint32_t acc)
@@ -117,21 +118,25 @@ __device__ __forceinline__ void mma_tf32(uint32_t d, uint64_t a, uint64_t b, uin
         "l"(a), "l"(b), "r"(id), "r"(acc));
 }
 
+__device__ __forceinline__ bool mbar_try(uint32_t mbar, uint32_t parity)
+{
+    uint32_t ok;
+    asm volatile(
+        "{\n"
+        ".reg .pred P;\n"
+        "mbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2;\n"
+        "selp.b32 %0, 1, 0, P;\n"
+        "}\n"
+        : "=r"(ok)
+        : "r"(mbar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+
 __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity, uint32_t limit)
 {
-    for (uint32_t i = 0; i < limit; i++) {
-        uint32_t ok;
-        asm volatile(
-            "{\n"
-            ".reg .pred P;\n"
-            "mbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2;\n"
-            "selp.b32 %0, 1, 0, P;\n"
-            "}\n"
-            : "=r"(ok)
-            : "r"(mbar), "r"(parity)
-            : "memory");
-        if (ok) return true;
-    }
+    for (uint32_t i = 0; i < limit; i++)
+        if (mbar_try(mbar, parity)) return true;
     return false;
 }
 
@@ -286,8 +291,7 @@ __device__ __forceinline__ void product_issue(const ctx& c)
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     fence_before();
     __syncthreads();
-    // (*fail is set in product_wait, before this barrier)
-    if (threadIdx.x == 0 && *c.fail == 0) {
+    if (threadIdx.x == 0 && c.live) {
         fence_after();
         constexpr uint32_t id = idesc<V>();
 #pragma unroll
@@ -313,18 +317,29 @@ __device__ __forceinline__ void product_issue(const ctx& c)
     }
 }
 
-// The vote makes the warp whole again after the polling loop, whose lanes
-// leave it one by one: the TMEM loads that follow are warp-wide
-// (.sync.aligned). False, for the whole warp, where the product is not known
-// to be complete: its accumulators are not to be read.
-__device__ __forceinline__ bool product_wait(ctx& c)
+// The issuing thread's warp alone decides whether a next product is issued:
+// if it saw this one complete, none is outstanding. The others look at *fail
+// while they poll, so that no warp waits long for a product that never comes.
+// __syncwarp: the polling loop's lanes leave it one by one, and the TMEM loads
+// that follow are warp-wide (.sync.aligned). (After a time-out they read void
+// accumulators into void results; skipping them would keep the compiler from
+// loading the coefficients behind the wait: 6 levels, 2.5 % of the step.)
+__device__ __forceinline__ void product_wait(ctx& c)
 {
-    const bool ok = *c.fail == 0 && mbar_wait(c.mbar, c.phase, c.wait_limit);
-    if (!ok) *c.fail = 1;
+    if (c.live) {
+        bool ok = false;
+        for (uint32_t i = 0; i < c.wait_limit; i++) {
+            ok = mbar_try(c.mbar, c.phase);
+            if (ok || ((i & 63u) == 63u && *c.fail != 0)) break;
+        }
+        if (!ok) {
+            c.live = false;
+            *c.fail = 1;
+        }
+    }
     c.phase ^= 1u;
-    const bool all = __all_sync(0xffffffffu, ok);
+    __syncwarp();
     fence_after();
-    return all;
 }
 
 // Row threadIdx.x of D0 and D1 (FIX: of D0 and of the sum of the others), 16
@@ -397,7 +412,7 @@ __device__ __forceinline__ void rotate_df(float (&uh)[V], float (&ul)[V], float 
 // on the tensor cores. The product reads its own copy of the vector
 // (shared memory), so the registers are updated in place. All threads of
 // the CTA call it (threads without a point pass zeros and discard the
-// result). pout stays as it was when the product did not complete.
+// result).
 template<int V, class CF>
 __device__ __forceinline__ void cvr_update_df_tc(
     ctx& c, float (&uh)[V], float (&ul)[V], float e, float& pout, const CF& cf)
@@ -405,7 +420,7 @@ __device__ __forceinline__ void cvr_update_df_tc(
     rotate_df<V>(uh, ul, e, cf);
     write_row<V>(c, uh);
     product_issue<V>(c);
-    if (!product_wait(c)) return;
+    product_wait(c);
     float pp = cf.p0();
     consume_row<V>(c, [&](auto I, float d, float dl) {
         constexpr int i = decltype(I)::value;
@@ -435,7 +450,7 @@ __device__ __forceinline__ void cayley_update_df_tc(
     product_issue<NN, true>(c);
     float inc[NN];
     cayley_increment_df<N>(rh, e, cf, inc);
-    if (!product_wait(c)) return;
+    product_wait(c);
     float acc = 0.0f;
     consume_row<NN, true>(c, [&](auto I, float d, float dl) {
         constexpr int i = decltype(I)::value;

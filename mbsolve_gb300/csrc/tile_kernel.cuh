@@ -154,7 +154,7 @@ struct tile_own {
     uint32_t bits;  // sources (bits 0 ..), records (bits 8 ..); OWN_ALL: more than a tile lists
     int32_t src;    // -1, or the only source: first value | point << 16 | type << 24
     int32_t rec;    // -1, or the field record: index | point << 8 | type << 16
-    uint32_t left;  // its rows from here on
+    uint32_t left;  // its rows from here on (not 0 while its bit is set)
     T* dst;         // its next row
 };
 
@@ -182,14 +182,15 @@ __device__ __forceinline__ tile_own<T> own_lists(const kparams<T>& p, const tile
         const int64_t lo = max((int64_t) rc.pos, (int64_t) td.out_start);
         const int64_t hi = min((int64_t) rc.pos + rc.cols, (int64_t) td.out_start + td.out_len);
         if (l0 + C <= lo || l0 >= hi) continue;
-        own.bits |= 256u << r;
         if (own.rec < 0 && rc.cols == 1 && rc.type <= 2) {
             // the row of the launch's first due step
             const uint64_t row = tl.row0[r] + (tl.mask[r][0] & 1u ? 0u : 1u);
+            if (row >= rc.rows) continue;  // steps due beyond the last row take none
             own.rec = r | (int) (lo - l0) << 8 | rc.type << 16;
             own.dst = p.scratch + rc.offset + row;
-            own.left = row < rc.rows ? (uint32_t) min(rc.rows - row, (uint64_t) 0xffffffffu) : 0u;
+            own.left = (uint32_t) min(rc.rows - row, (uint64_t) 0xffffffffu);
         }
+        own.bits |= 256u << r;
     }
     return own;
 }
@@ -252,14 +253,9 @@ __device__ __forceinline__ void for_records(const kparams<T>& p, const run_desc&
         if (todo & bit) {
             todo &= ~bit;
             const T v = field((own.rec >> 8) & 255, own.rec >> 16);
-            // (a step may be due beyond the last row; it is no part of the
-            // results)
-            if (own.left) {
-                *own.dst = v;
-                if (!isfinite(v)) atomicOr(p.status, STATUS_NONFINITE);
-                own.left--;
-            }
-            own.dst++;
+            *own.dst++ = v;
+            if (--own.left == 0u) own.bits &= ~(256u << (own.rec & 255));
+            if (!isfinite(v)) atomicOr(p.status, STATUS_NONFINITE);
         }
         if (todo == 0u) return;
     }
@@ -839,7 +835,8 @@ __device__ __forceinline__ void step_body(const kparams<T>& p, uint32_t tile, ui
         tcc.phase = *res.phase;
         tcc.wait_limit = p.tc_stall ? 0u : p.wait_limit ? p.wait_limit : tc::WAIT_LIMIT;
         tcc.fail = res.fail;
-        if (uniform && *tcc.fail == 0) {
+        tcc.live = *res.fail == 0;
+        if (uniform && tcc.live) {
             const T* mat = p.mc + (uint64_t) td.uniform_mat * p.mstride;
             if constexpr (ALGO == 1) {
                 tc::stage_b<D>(tcc, mat + pre::FDTD_END, mat + pre::FDTD_END + D * D, D);
