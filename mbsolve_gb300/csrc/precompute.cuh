@@ -567,8 +567,8 @@ MBG_HD void jacobi_hermitian(
 
 // The same by one thread, a matrix's columns, its rows and the eigenvectors'
 // columns in loops of their own: the loops above, as a group of one, took
-// 2.13 s instead of 1.84 for 16,384 6-level materials (one thread each, at the
-// memory's rate) and 0.69 instead of 0.67 for 128.
+// 0.3 s more for 16,384 6-level materials (1.74 s, one thread each, at the
+// memory's rate) and 3 % more for 128.
 MBG_HD void jacobi_hermitian(
     double* are,
     double* aim,
@@ -856,7 +856,13 @@ MBG_HD int cvr_precompute(const mat_in& m, int Nsolver, double* ws, double* out,
     }
     // relaxation superoperator G_ij = Re 1/2 tr(R(g_j) g_i) and the
     // equilibrium vector d_eq_i = Re tr(R(I) g_i) / N (cvr.hpp:181-213)
-    double tre[36], tim[36], ure[36], uim[36];
+    // (each thread's four N x N scratch matrices in the workspace, not its
+    // stack: a kernel whose stack frame exceeds the context's limit of 1,024
+    // bytes makes the driver allocate when it is launched)
+    double* tre = F + (size_t) (g.rank < V ? g.rank : 0) * 4 * NN;  // 4 V NN <= 9 V V
+    double* tim = tre + NN;
+    double* ure = tim + NN;
+    double* uim = ure + NN;
     for (int j = g.rank; j < V; j += g.size) {
         int nz = generator_entries(N, j, gr, gc, gv);
         for (int e = 0; e < NN; e++) tre[e] = tim[e] = 0.0;
@@ -871,14 +877,16 @@ MBG_HD int cvr_precompute(const mat_in& m, int Nsolver, double* ws, double* out,
             M[i * V + j] += 0.5 * t.re;
         }
     }
-    for (int e = 0; e < NN; e++) {
-        tre[e] = (e % (N + 1) == 0) ? 1.0 : 0.0;
-        tim[e] = 0.0;
-    }
-    relax_apply(m, tre, tim, ure, uim);
-    for (int i = g.rank; i < V; i += g.size) {
-        int nz = generator_entries(N, i, gr, gc, gv);
-        d_eq[i] = trace_with_gen(ure, uim, N, nz, gr, gc, gv).re / N;
+    if (g.rank < V) {
+        for (int e = 0; e < NN; e++) {
+            tre[e] = (e % (N + 1) == 0) ? 1.0 : 0.0;
+            tim[e] = 0.0;
+        }
+        relax_apply(m, tre, tim, ure, uim);
+        for (int i = g.rank; i < V; i += g.size) {
+            int nz = generator_entries(N, i, gr, gc, gv);
+            d_eq[i] = trace_with_gen(ure, uim, N, nz, gr, gc, gv).re / N;
+        }
     }
     g.sync();
     const double M_CP = 0.5 * m.carrier_density;
