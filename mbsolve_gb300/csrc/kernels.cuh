@@ -82,8 +82,9 @@ struct kparams {
 // ------------------------------------------------------------ helpers
 
 // sin(x) and 1 - cos(x). For small |x| by their Taylor series (enough
-// terms for the type's precision: truncation below 1e-10 relative in
-// float, 1e-30 in double); beyond that by the library sincos.
+// terms for the type's precision: the first omitted terms are below 4e-11
+// of the result in float, 1e-17 in double); beyond that by the library
+// sincos.
 template<typename T>
 __device__ __forceinline__ void rot_coeffs(T x, T& s, T& s2);
 
@@ -124,11 +125,11 @@ __device__ __forceinline__ void rot_coeffs<float>(float x, float& s, float& s2)
 // Horner form by compile-time reciprocals (a division takes ten
 // instructions), as many terms as the range needs: for |x| < 2^-6 (fields up
 // to ten times the strongest of the presets) the first omitted terms are
-// below 2^-65 of the result, for |x| < 1/4 below 1e-17; 10 and 18
+// below 2^-65 of the result, for |x| < 1/4 below 1e-17; 9 and 15
 // instructions. The range is read from the exponent bits: an FP64 compare
 // would be one more. With the 20 divisions of a recurrence before, a 2-level
 // point and step took 193 FP64 instructions; now about 30 (2-level preset,
-// 32,768 points, 10,000 steps: 165.6 -> 33.4 ms; 6 levels, 65,536 points: 9.5e7 ->
+// 32,768 points, 10,000 steps: 165.9 -> 31.1 ms; 6 levels, 65,536 points: 9.5e7 ->
 // 3.2e8 cell-updates/s, the unit's rate for the 1,225 products of a step).
 template<>
 __device__ __forceinline__ void rot_coeffs<double>(double x, double& s, double& s2)

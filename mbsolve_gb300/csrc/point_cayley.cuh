@@ -19,9 +19,10 @@ namespace mbg {
 
 constexpr int POINT_THREADS = 32;
 
-// 1 / x by two Newton steps from an FP32 reciprocal (22 -> 44 -> 88 bits, the
-// last rounded to FP64: within an ulp): 4 FP64 instructions instead of a
-// division's ten. FP32 and back through the bits, because a conversion is
+// 1 / x by two Newton steps from an FP32 reciprocal (21 -> 42 -> 84 bits, the
+// last rounded to FP64: the division's result, unless the quotient lies within
+// 2^-31 of an ulp of the middle between two numbers): 4 FP64 instructions
+// instead of a division's ten. FP32 and back through the bits, because a conversion is
 // an FP64 instruction too. x is the squared modulus of a pivot of I + iK,
 // whose Hermitian part is I: at least 1; beyond FP32's range the division.
 __device__ __forceinline__ double pivot_reciprocal(double x)
