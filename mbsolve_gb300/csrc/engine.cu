@@ -1530,6 +1530,17 @@ private:
     // changes with the set of kernels, so that a file's entries of another
     // set are not read.
     static constexpr const char* TUNE_SET = "k2";
+    // Shape and depth are tuned together up to here. Single runs, us a step,
+    // one after the other / together:
+    //   2 levels FP32     4,096 0.59 / 0.56, 16,384 0.63 / 0.59, 131,072 1.22 / 1.12,
+    //                     200,000 1.59 / 1.58, 500,000 4.9 / 6.1
+    //   2 levels FP64     131,072 11.0 / 10.7, 500,000 32.7 / 32.5
+    //   3-level Cayley    50,000 3.17 / 3.02, 131,072 6.57 / 5.77, 200,000 9.7 / 8.8,
+    //                     500,000 24.7 to 26.6 / 24.4
+    //   6 levels FP32     1,000 to 500,000 within 1 %
+    // (5-level FP64 Cayley within 0.1 %; 100 and 1,000 2-level points within 1 %).
+    // Above, the pick at the depth timed need not be the persistent kernel's
+    // best, and the search takes up to twice as long (0.18 -> 0.29 s).
     static constexpr uint64_t JOINT_CELLS = 1u << 17;
 
     std::string tune_key(int forced) const
