@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(POINT_THREADS) point_cayley_kernel(const kpara
     double xi = i == j ? 0.0 : sg * p.Din[(uint64_t) (at + 1) * p.plane + g0];
 
     __syncwarp();
-    tile_own<double> own{ 0u, -1, -1, 0u, nullptr };
+    tile_own<double> own{ 0u, -1, -1, nullptr };
     if (tl.nsrc + tl.nrec > 0 || tl.overflow) {
         prepare_lists<double, POINT_THREADS>(p, tl, sv, step0, nsteps);
         __syncwarp();

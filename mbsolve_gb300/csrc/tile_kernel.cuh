@@ -154,7 +154,6 @@ struct tile_own {
     uint32_t bits;  // sources (bits 0 ..), records (bits 8 ..); OWN_ALL: more than a tile lists
     int32_t src;    // -1, or the only source: first value | point << 16 | type << 24
     int32_t rec;    // -1, or the field record: index | point << 8 | type << 16
-    uint32_t left;  // its rows from here on (not 0 while its bit is set)
     T* dst;         // its next row
 };
 
@@ -163,7 +162,7 @@ template<typename T, int C>
 __device__ __forceinline__ tile_own<T> own_lists(const kparams<T>& p, const tile_lists& tl, const tile_desc& td,
                                                  int64_t l0, int nsteps)
 {
-    tile_own<T> own{ 0u, -1, -1, 0u, nullptr };
+    tile_own<T> own{ 0u, -1, -1, nullptr };
     if (tl.overflow) {
         own.bits = OWN_ALL;
         return own;
@@ -182,15 +181,15 @@ __device__ __forceinline__ tile_own<T> own_lists(const kparams<T>& p, const tile
         const int64_t lo = max((int64_t) rc.pos, (int64_t) td.out_start);
         const int64_t hi = min((int64_t) rc.pos + rc.cols, (int64_t) td.out_start + td.out_len);
         if (l0 + C <= lo || l0 >= hi) continue;
-        if (own.rec < 0 && rc.cols == 1 && rc.type <= 2) {
-            // the row of the launch's first due step
-            const uint64_t row = tl.row0[r] + (tl.mask[r][0] & 1u ? 0u : 1u);
-            if (row >= rc.rows) continue;  // steps due beyond the last row take none
-            own.rec = r | (int) (lo - l0) << 8 | rc.type << 16;
-            own.dst = p.scratch + rc.offset + row;
-            own.left = (uint32_t) min(rc.rows - row, (uint64_t) 0xffffffffu);
-        }
         own.bits |= 256u << r;
+        // (steps due beyond the record's last row, which take none, are left
+        // to for_records' general part: a count of the rows left would cost
+        // every thread of the loop)
+        if (own.rec < 0 && rc.cols == 1 && rc.type <= 2 && nsteps > 0 && tl.row(r, nsteps - 1) < rc.rows) {
+            own.rec = r | (int) (lo - l0) << 8 | rc.type << 16;
+            // the row of the launch's first due step
+            own.dst = p.scratch + rc.offset + tl.row0[r] + (tl.mask[r][0] & 1u ? 0u : 1u);
+        }
     }
     return own;
 }
@@ -254,7 +253,6 @@ __device__ __forceinline__ void for_records(const kparams<T>& p, const run_desc&
             todo &= ~bit;
             const T v = field((own.rec >> 8) & 255, own.rec >> 16);
             *own.dst++ = v;
-            if (--own.left == 0u) own.bits &= ~(256u << (own.rec & 255));
             if (!isfinite(v)) atomicOr(p.status, STATUS_NONFINITE);
         }
         if (todo == 0u) return;
@@ -810,7 +808,7 @@ __device__ __forceinline__ void step_body(const kparams<T>& p, uint32_t tile, ui
         }
     }
     __syncthreads();
-    tile_own<T> own{ 0u, -1, -1, 0u, nullptr };
+    tile_own<T> own{ 0u, -1, -1, nullptr };
     if (tl.nsrc + tl.nrec > 0 || tl.overflow) {  // the same in every thread
         prepare_lists<T, NT>(p, tl, sv, step0, nsteps);
         __syncthreads();
