@@ -1710,7 +1710,7 @@ private:
         if (t.depth < 1 || t.depth > MAX_DEPTH) throw invalid_argument("temporal depth must be 1..256");
         // Runs of a single grid point, FP64 Cayley, no launch shape asked
         // for: one warp per point over as many steps as a launch can hold
-        // (3-level preset, 10,000 steps: 52 ms against 188 with a
+        // (3-level preset, 10,000 steps: 51 ms against 188 with a
         // point per lane). There is nothing to tune.
         bool point = staging_ == STAGING_REGS && !(user && (user->cells_per_thread || user->threads || user->depth));
         for (const auto& r : runs_) point = point && r.n_x == 1;

@@ -8,7 +8,7 @@
 // other. With the entry (i, j) of every N x N matrix in lane i N + j a
 // product is 4 N of them, and the solve A Y = K runs by Gauss-Jordan
 // elimination, which updates all rows of a column at once: about 125 FP64
-// instructions (3-level preset, 10,000 steps: 188 -> 52 ms).
+// instructions (3-level preset, 10,000 steps: 188 -> 51 ms).
 // The state in memory, the steps per launch, sources and records are those
 // of the tile kernels (cayley_update has the formulas).
 #pragma once
